@@ -168,6 +168,33 @@ inline size_t cell(const AtjupCtx* c, int i, int j, int k) {
     return ((size_t)i * c->P.jm + j) * c->KP + k;
 }
 
+// Programmatic dependent launch: a kernel launched by launch_pdl may start while the kernel before it
+// on the stream is finishing (from when each of that one's blocks has called pdl_next or ended); it
+// must call pdl_wait before it reads or writes anything the stream's earlier work touches -- the wait
+// ends when that work is complete and visible. What a kernel does before pdl_wait (index arithmetic,
+// loads of constants) and its launch latency then overlap the tail of the one before.
+__device__ __forceinline__ void pdl_next() {
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+// With overlap false the launch is an ordinary one (pdl_wait returns at once).
+template <typename... P, typename... A>
+cudaError_t launch_pdl(bool overlap, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                       cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // launchers (return ATJUP_OK or an error code)
 int launch_buoy_ref(AtjupCtx* c, const double* t);
 int launch_hydrostatic(AtjupCtx* c, const double* v, const double* w);

@@ -24,7 +24,6 @@ namespace {
 // The tiles cover the km-1 = 360 distinct meridians exactly (10 x 36); the seam copy k = km-1 is
 // never read by a stage (the ring wraps 359 -> 0) and is left alone.
 constexpr int TK = 36, TJ = 7, NT = 256, NL = TK * TJ;   // 252 live threads of 256
-constexpr int NCH = 2;   // radial chunks per column tile (the step: 6.69 ms, 6.72 with 3 or 4)
 constexpr int HJ = TJ + 2;                               // halo rows of a tile
 constexpr int NX = 5;    // FP64 per-cell inputs besides Y: rho, wall_nue, nue, Q_rad, Q_precip
 
@@ -37,6 +36,7 @@ enum : uint8_t { NB_S = 1, NB_IP = 2, NB_IM = 4, NB_JP = 8, NB_JM = 16, NB_KP = 
 struct StageConst {
     int im, jm, km, KP;
     int stage;
+    int per;                   // radial planes per block
     double c_in, wgt, dt, one_sixth;
     double inv_2dr, inv_2dthe, inv_2dphi, inv_dr2, inv_dthe2, inv_dphi2;
     double cor_phi_f;          // (nd_cor * 2) * omega
@@ -299,7 +299,7 @@ rk_stage_kernel(StagePtrs a, StageConst q, const __grid_constant__ StageMaps M) 
     const int hT = (ty + 1) * WT + (tx + Box3<TI>::OX);      // this cell in a stage-input box
     const int hP = (ty + 1) * WP + (tx + Box3<double>::OX);  // this cell in a pressure box
     // radial chunk [i_lo, i_hi); the march starts one plane below to fill the radial window
-    const int per = (q.im + NCH - 1) / NCH;
+    const int per = q.per;
     const int i_lo = blockIdx.z * per, i_hi = min(q.im, i_lo + per);
     const int i_st = (i_lo > 0) ? i_lo - 1 : 0;
     const int role = wrap_role(tid, k0, q);
@@ -778,6 +778,19 @@ static int make_box_map(CUtensorMap* m, const void* base, const AtjupCtx* c, int
     return ATJUP_OK;
 }
 
+// Radial planes per block of the stage kernel. A block's planes are a chain (3.7 us each when it has an
+// SM to itself), so a grid is cut into chunks short enough that every SM has its two blocks, down to
+// two planes (each chunk reads the two planes beside it again, from L2): 41x61x97, 27 tiles, 79 us a
+// stage in two chunks and 25 us in chunks of 4; 13x37x49, 12 tiles, 26 and 13 us. Grids that fill the
+// chip anyway take 8: chunks of 6 to 14 measured alike there (41x181x361: two dry iterations 1.80 to
+// 1.83 ms, 1.92 in two chunks, 2.01 in chunks of 2).
+static int planes_per_block(const AtjupParams& P) {
+    const long tiles = (long)((P.km - 1 + TK - 1) / TK) * ((P.jm + TJ - 1) / TJ);
+    int per = 8;
+    while (per > 2 && tiles * ((P.im + per - 1) / per) < 2 * 148) per--;
+    return per;
+}
+
 template <typename TI, typename TO, typename TA, typename R>
 static int launch_stage_t(AtjupCtx* c, const StagePtrs& a, const StageConst& q, const char* name) {
     const AtjupParams& P = c->P;
@@ -810,7 +823,7 @@ static int launch_stage_t(AtjupCtx* c, const StagePtrs& a, const StageConst& q, 
                 if (int rc = make_box_map<TA>(&M.ax[f], src[f], c, TK, TJ)) return rc;
         }
     }
-    dim3 grid((P.km - 1 + TK - 1) / TK, (P.jm + TJ - 1) / TJ, NCH);
+    dim3 grid((P.km - 1 + TK - 1) / TK, (P.jm + TJ - 1) / TJ, (P.im + q.per - 1) / q.per);
     c->launches++;
     rk_stage_kernel<TI, TO, TA, R><<<grid, NT, sizeof(StageSmem<TI, TA>), c->stream>>>(a, q, M);
     ATJUP_CHECK_LAUNCH(name);
@@ -851,6 +864,7 @@ int launch_rk_stage(AtjupCtx* c, int stage, const void* const* Xin, void* const*
     StageConst q{};
     q.im = P.im; q.jm = P.jm; q.km = P.km; q.KP = c->KP;
     q.stage = stage;
+    q.per = planes_per_block(P);
     q.c_in = (stage == 0 || stage == 1) ? 0.5 * P.dt : (stage == 2 ? P.dt : 0.0);
     q.wgt = (stage == 0 || stage == 3) ? 1.0 : 2.0;
     q.dt = P.dt;

@@ -125,7 +125,7 @@ void free_all(AtjupCtx* c) {
     cudaFree(c->mca_pairs);
     cudaFree(c->solve_b); cudaFree(c->dsum); cudaFree(c->counters);
     if (c->hsum) cudaFreeHost(c->hsum);
-    cudaFree(c->solid); cudaFree(c->nbflags); cudaFree(c->topo); cudaFree(c->geo); cudaFree(c->cor_col);
+    cudaFree(c->solid); cudaFree(c->nbflags); cudaFree(c->topo); cudaFree(c->floor_hi); cudaFree(c->run); cudaFree(c->geo); cudaFree(c->cor_col);
     cudaFree(c->sin_the); cudaFree(c->rad); cudaFree(c->cell_vbar0); cudaFree(c->cell_ubar0);
     cudaFree(c->solid_list); cudaFree(c->amb_rows); cudaFree(c->yw);
     cudaFree(c->line_a); cudaFree(c->line_c); cudaFree(c->line_m);
@@ -395,6 +395,22 @@ int atjup_gpu_set_grid(AtjupCtx* c, const double* rad, const double* the, const 
     ATJUP_CUDA(cudaMemcpy(c->cor_col, cor_col.data(), sizeof(double) * jm, cudaMemcpyHostToDevice));
     ATJUP_CUDA(cudaMemcpy(c->sin_the, sin_the.data(), sizeof(double) * jm, cudaMemcpyHostToDevice));
     ATJUP_CUDA(cudaMemcpy(c->rad, rad, sizeof(double) * im, cudaMemcpyHostToDevice));
+    if (int rc = filter_tables(c, i_topo)) return rc;
+    // per column the run of fluid cells above its foot: [x, y], x = im (y = im - 1) when it has none
+    std::vector<int2> run((size_t)jm * KP, make_int2(im, im - 1));
+    std::vector<uint8_t> done((size_t)jm * km, 0);          // 0 below the run, 1 in it, 2 above
+    for (int i = 0; i < im; i++)
+        for (int j = 0; j < jm; j++) {
+            const uint8_t* s = solid + ((size_t)i * jm + j) * km;
+            uint8_t* d = &done[(size_t)j * km];
+            int2* r = &run[(size_t)j * KP];
+            for (int k = 0; k < km; k++) {
+                if (!s[k] && d[k] == 0) { d[k] = 1; r[k].x = i; }
+                else if (s[k] && d[k] == 1) { d[k] = 2; r[k].y = i - 1; }
+            }
+        }
+    if (!c->run) ATJUP_CUDA(cudaMalloc(&c->run, sizeof(int2) * run.size()));
+    ATJUP_CUDA(cudaMemcpy(c->run, run.data(), sizeof(int2) * run.size(), cudaMemcpyHostToDevice));
     cudaFree(c->cell_vbar0); cudaFree(c->cell_ubar0);
     c->cell_vbar0 = c->cell_ubar0 = nullptr;
     if (cell_vbar0 && cell_ubar0) {
@@ -629,7 +645,7 @@ int atjup_gpu_set_physics(AtjupCtx* c, const AtjupPhysics* ph, const float* laye
         A(&c->S2[s], c->NP);
         A(&c->Sacc[s], c->NP);
     }
-    if (rc) return rc;
+    if (rc || (rc = side_init(c))) return rc;
     if (!c->layer_h) ATJUP_CUDA(cudaMalloc(&c->layer_h, sizeof(float) * P.im));
     ATJUP_CUDA(cudaMemcpy(c->layer_h, layer_heights_km, sizeof(float) * P.im,
                           cudaMemcpyHostToDevice));
@@ -730,15 +746,17 @@ int atjup_gpu_download_n(AtjupCtx* c, int32_t id, double* host) {
     return ATJUP_OK;
 }
 
+// restoreVar of every transported scalar, after the clamp of the first n_clamp (the species come first)
+static int restore_all(AtjupCtx* c, int n_clamp) {
+    int idx[ATJUP_S_COUNT + 2];
+    for (int s = 0; s < ATJUP_S_COUNT + 2; s++) idx[s] = s;
+    return launch_sync_n(c, idx, ATJUP_S_COUNT + 2, n_clamp);
+}
+
 int atjup_gpu_restore_scalars(AtjupCtx* c) {
     if (!c) { set_error("restore_scalars: null context"); return ATJUP_ERR_ARG; }
     if (!c->phys_on) return ATJUP_OK;
-    for (int s = 0; s < ATJUP_S_COUNT + 2; s++) {
-        const int id = kScalarField[s];
-        ATJUP_CUDA(cudaMemcpyAsync(c->fn[id], c->f[id], c->NP * sizeof(double),
-                                   cudaMemcpyDeviceToDevice, c->stream));
-    }
-    return ATJUP_OK;
+    return restore_all(c, 0);
 }
 
 int atjup_gpu_upload2d(AtjupCtx* c, int32_t id, const double* host) {
@@ -854,16 +872,6 @@ int atjup_gpu_balance_column_v(AtjupCtx* c, double* vshift) {
 }
 
 namespace {
-// live -> time-level-n copy of the transported scalars with the given ATJUP_S_* indices
-int copy_to_n(AtjupCtx* c, const int* idx, int n) {
-    for (int q = 0; q < n; q++) {
-        const int id = kScalarField[idx[q]];
-        ATJUP_CUDA(cudaMemcpyAsync(c->fn[id], c->f[id], c->NP * sizeof(double),
-                                   cudaMemcpyDeviceToDevice, c->stream));
-    }
-    return ATJUP_OK;
-}
-
 // The physics part of the even iterations (cJupiterModel.cpp:1054-1162): radiation, the three
 // saturation adjustments, the NH4SH equilibrium, precipitation, the scalar sync of
 // ATJUP_RK_SCALAR_SYNC = 2 (t needs none: its time-level-n copy is the live field on the
@@ -894,7 +902,7 @@ int physics_block(AtjupCtx* c) {
         const int sync[11] = {ATJUP_S_H2O, ATJUP_S_H2O_CLOUD, ATJUP_S_H2O_ICE, ATJUP_S_NH3,
                               ATJUP_S_NH3_CLOUD, ATJUP_S_NH3_ICE, ATJUP_S_CH4, ATJUP_S_CH4_CLOUD,
                               ATJUP_S_CH4_ICE, ATJUP_S_H2S, ATJUP_S_NH4SH};
-        if ((rc = copy_to_n(c, sync, mc.nh4sh_eq ? 11 : 9))) return rc;
+        if ((rc = launch_sync_n(c, sync, mc.nh4sh_eq ? 11 : 9, 0))) return rc;
     }
     if (c->phys.turb_on && (rc = atjup_gpu_turbulence(c))) return rc;
     if (c->micro_on && (rc = atjup_gpu_chemistry(c))) return rc;
@@ -932,8 +940,9 @@ int atjup_gpu_step(AtjupCtx* c, int32_t iter_n, int32_t first, const AtjupSolveO
         if ((rc = launch_mca(c))) return rc;
     }
     if (P.shapiro_inloop > 0) {
-        for (int f = ATJUP_F_U; f <= ATJUP_F_W; f++)
-            if ((rc = atjup_gpu_shapiro(c, f, 4, P.shapiro_strength, P.shapiro_inloop, 1))) return rc;
+        Timed tm(c, TK_SHAPIRO);
+        if ((rc = launch_shapiro_n(c, &c->f[ATJUP_F_U], 3, 4, P.shapiro_strength, P.shapiro_inloop, 1)))
+            return rc;
     }
     if (P.v_massbal_stride > 0 && iter_n % P.v_massbal_stride == 0) {
         Timed tm(c, TK_BALANCE_V);
@@ -947,8 +956,9 @@ int atjup_gpu_step(AtjupCtx* c, int32_t iter_n, int32_t first, const AtjupSolveO
     if (mca_now && (rc = join_side(c))) return rc;
     if (ph) {
         // clampNegativeSpecies, then restoreVar of the scalars (the dynamics need none)
-        if (c->micro_on && (rc = atjup_gpu_clamp_species(c))) return rc;
-        if ((rc = atjup_gpu_restore_scalars(c))) return rc;
+        if (c->micro_on && (rc = micro_supported(c))) return rc;
+        Timed tm(c, TK_MICRO);
+        if ((rc = restore_all(c, c->micro_on ? ATJUP_S_COUNT : 0))) return rc;
     }
     return ATJUP_OK;
 }

@@ -121,6 +121,8 @@ struct AtjupCtx {
     uint8_t* solid = nullptr;
     uint8_t* nbflags = nullptr;    // per-cell neighbour-solid and integrated flags (rk4.cu)
     int32_t* topo = nullptr;
+    int2* run = nullptr;           // [jm * KP]: the column's first fluid cell and the end of its run
+    int32_t* floor_hi = nullptr;   // [2 * jm * KP]: the filters' highest neighbour floors (filters.cu)
     atjup::GeoIJ* geo = nullptr;   // [im * jm]
     double* cor_col = nullptr;     // [jm] Coriolis factor of the hydrostatic integral
     double* sin_the = nullptr;     // [jm] sin(the_j), the area weight of the level mean
@@ -222,6 +224,9 @@ int rk4_tlm_ext(AtjupCtx* c, double* const d[4], const double* dp, const double*
 int rk4_adjoint_ext(AtjupCtx* c, double* const a[4], double* lp, double* lrho,
                     double* const laux[3], const double* const* stages = nullptr);
 int launch_shapiro(AtjupCtx* c, double* f, int order, double strength, int passes, int use_topo);
+int launch_shapiro_n(AtjupCtx* c, double* const* f, int n, int order, double strength, int passes,
+                     int use_topo);   // n <= 3 fields at once
+int filter_tables(AtjupCtx* c, const int32_t* topo);
 int launch_balance_v(AtjupCtx* c);
 int cone_prepare(AtjupCtx* c);
 int launch_cone_projection(AtjupCtx* c);
@@ -241,6 +246,8 @@ int launch_turbulence(AtjupCtx* c);
 int launch_turb_wall_hold(AtjupCtx* c);
 enum { MICRO_RADIATION = 0, MICRO_PRECIP, MICRO_NH4SH, MICRO_CHEMISTRY, MICRO_CLAMP, MICRO_DIAG };
 int launch_micro(AtjupCtx* c, int what);
+int micro_supported(const AtjupCtx* c);
+int launch_sync_n(AtjupCtx* c, const int* idx, int n, int n_clamp);
 int pressure_residual_solve(AtjupCtx* c, const AtjupSolveOpts* o, AtjupSolveStats* st);
 void solver_free(AtjupCtx* c);
 

@@ -867,8 +867,7 @@ int atjup_gpu_iteration_tlm(AtjupCtx* c, int32_t iter_n, int32_t first, int32_t 
         (rc = launch_bc_ptrs(c, ATJUP_BC_ALL, d[LT], d[LU], d[LV], d[LW], d[LP], S.pstat, false)))
         return rc;
     if ((parts & ATJUP_LIN_SHAPIRO) && P.shapiro_inloop > 0) {
-        for (int f = LU; f <= LW; f++)
-            if ((rc = launch_shapiro(c, d[f], 4, P.shapiro_strength, P.shapiro_inloop, 1))) return rc;
+        if ((rc = launch_shapiro_n(c, d + LU, 3, 4, P.shapiro_strength, P.shapiro_inloop, 1))) return rc;
     }
     if ((parts & ATJUP_LIN_BALANCE) && P.v_massbal_stride > 0 && iter_n % P.v_massbal_stride == 0) {
         if ((rc = launch_balance_v_buffers(d[LV], c->topo, c->rad, c->dvc, c->dvrow, P.im, P.jm,

@@ -462,6 +462,32 @@ __global__ void clamp_species_kernel(MicroArgs a) {
         if (!(a.q[s][c] >= 0.0)) a.q[s][c] = 0.0;
 }
 
+// live -> time-level-n copies of a list of transported scalars, the negative (or NaN) values of the
+// first n_clamp of them set to 0 in both (clampNegativeSpecies). One pass over the fields in place of a
+// pass that clamps and a copy per field; bound by memory (16 B per cell and field).
+struct SyncArgs {
+    double* live[ATJUP_S_COUNT + 2];
+    double* n[ATJUP_S_COUNT + 2];
+    int n_clamp;
+    size_t N;
+};
+__global__ void __launch_bounds__(256) sync_n_kernel(const __grid_constant__ SyncArgs a) {
+    double *x = a.live[blockIdx.y], *y = a.n[blockIdx.y];
+    const bool clamp = (int)blockIdx.y < a.n_clamp;
+    const size_t c = 4 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);      // rows are multiples of 16
+    if (c >= a.N) return;
+    double2 v0 = *reinterpret_cast<const double2*>(x + c);
+    double2 v1 = *reinterpret_cast<const double2*>(x + c + 2);
+    if (clamp) {
+        if (!(v0.x >= 0.0)) x[c] = v0.x = 0.0;
+        if (!(v0.y >= 0.0)) x[c + 1] = v0.y = 0.0;
+        if (!(v1.x >= 0.0)) x[c + 2] = v1.x = 0.0;
+        if (!(v1.y >= 0.0)) x[c + 3] = v1.y = 0.0;
+    }
+    *reinterpret_cast<double2*>(y + c) = v0;
+    *reinterpret_cast<double2*>(y + c + 2) = v1;
+}
+
 // The output diagnostics: the force densities of Forces and the latent and sensible heating of
 // Latent_Heat. One thread per cell; both routines fill i 1..im-2, j 1..jm-2 and the phi ring
 // k 0..km-2, Latent_Heat also zeroes its fields at i = 0; other cells keep their values. The
@@ -619,12 +645,33 @@ MicroArgs make_args(AtjupCtx* c) {
 
 }  // namespace
 
-int launch_micro(AtjupCtx* c, int what) {
-    const AtjupParams& P = c->P;
-    if (P.im > MAX_IM) {
+// The time-level-n copies of the scalars with the ATJUP_S_* indices idx (ATJUP_S_COUNT, + 1: k*, omega*),
+// the first n_clamp of them clamped at 0 as well
+int launch_sync_n(AtjupCtx* c, const int* idx, int n, int n_clamp) {
+    SyncArgs a{};
+    for (int q = 0; q < n; q++) {
+        a.live[q] = c->f[kScalarField[idx[q]]];
+        a.n[q] = c->fn[kScalarField[idx[q]]];
+    }
+    a.n_clamp = n_clamp;
+    a.N = c->NP;
+    c->launches++;
+    sync_n_kernel<<<dim3((unsigned)((c->NP / 4 + 255) / 256), n), 256, 0, c->stream>>>(a);
+    ATJUP_CHECK_LAUNCH("sync_n");
+    return ATJUP_OK;
+}
+
+int micro_supported(const AtjupCtx* c) {
+    if (c->P.im > MAX_IM) {
         set_error("microphysics: more than 64 radial levels");
         return ATJUP_ERR_UNSUPPORTED;
     }
+    return ATJUP_OK;
+}
+
+int launch_micro(AtjupCtx* c, int what) {
+    const AtjupParams& P = c->P;
+    if (int rc = micro_supported(c)) return rc;
     MicroArgs a = make_args(c);
     const int TB = 128;
     const dim3 gcol((P.km + TB - 1) / TB, P.jm);
@@ -647,14 +694,12 @@ int launch_micro(AtjupCtx* c, int what) {
         difflux_kernel<<<gcell, TB, 0, c->stream>>>(a);
         c->launches++;
         ATJUP_CHECK_LAUNCH("difflux_kernel");
-        for (int q = 0; q < 3; q++)
-            if ((rc = launch_shapiro(c, a.difflux[q], 2, 1.0, 1, 1))) return rc;
+        if ((rc = launch_shapiro_n(c, a.difflux, 3, 2, 1.0, 1, 1))) return rc;
         massflux_kernel<<<gcell, TB, 0, c->stream>>>(a);
         fluxlim_kernel<<<gcell, TB, 0, c->stream>>>(a);
         c->launches += 2;
         ATJUP_CHECK_LAUNCH("massflux/fluxlim kernels");
-        for (int q = 0; q < 3; q++)
-            if ((rc = launch_shapiro(c, a.massflux[q], 2, 1.0, 1, 1))) return rc;
+        if ((rc = launch_shapiro_n(c, a.massflux, 3, 2, 1.0, 1, 1))) return rc;
         if ((rc = launch_shapiro(c, a.fluxlim, 2, 1.0, 1, 1))) return rc;
         break;
     }

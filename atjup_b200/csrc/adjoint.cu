@@ -490,10 +490,31 @@ __global__ void ad_stage_kernel(AdArgs A, LinConst q) {
     if ((threadIdx.x & 31) == 0 && lb_cell != 0.0) atomicAdd(A.lb + i, lb_cell);
 }
 
-// lY += lX over every cell of the padded block
-__global__ void add_kernel(double* __restrict__ y, const double* __restrict__ x, size_t n) {
+// lY += lX over every cell of the padded block, the four fields at once (blockIdx.y)
+struct AddArgs {
+    double* y[4];
+    const double* x[4];
+};
+__global__ void add_kernel(const __grid_constant__ AddArgs a, size_t n) {
     const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < n) y[c] += x[c];
+    if (c < n) a.y[blockIdx.y][c] += a.x[blockIdx.y][c];
+}
+
+// dst[f] = src[f] over the padded block, up to COPY_MAX fields at once (16-byte accesses: KP is a
+// multiple of 16, and the buffers' alignment is checked by the caller)
+constexpr int COPY_MAX = 9;
+struct CopyArgs {
+    double* dst[COPY_MAX];
+    const double* src[COPY_MAX];
+};
+__global__ void __launch_bounds__(256) copy_kernel(const __grid_constant__ CopyArgs a, size_t n) {
+    const size_t c = 4 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
+    if (c >= n) return;
+    const double* x = a.src[blockIdx.y] + c;
+    double* y = a.dst[blockIdx.y] + c;
+    const double2 u = *reinterpret_cast<const double2*>(x), v = *reinterpret_cast<const double2*>(x + 2);
+    *reinterpret_cast<double2*>(y) = u;
+    *reinterpret_cast<double2*>(y + 2) = v;
 }
 
 // ---- level mean: per level i, W_i = sum of sin(the_j) over the cells the forward mean counts
@@ -600,29 +621,55 @@ __global__ void tl_hydro_kernel(const double* __restrict__ v, const double* __re
     }
 }
 
-__global__ void ad_hydro_kernel(const double* __restrict__ v, const double* __restrict__ w,
-                                const double* __restrict__ lph, const uint8_t* __restrict__ solid,
-                                const double* __restrict__ rad, const double* __restrict__ cor_col,
-                                double* __restrict__ lv, double* __restrict__ lw, int im, int jm,
-                                int km, int KP, double dr) {
+// Eight levels' loads and divisions at a time: the running sum down the column only joins them (a level
+// at a time, with the mask read first, 73 us on 41x61x97).
+constexpr int AH = 8;
+__global__ void __launch_bounds__(64)
+ad_hydro_kernel(const double* __restrict__ v, const double* __restrict__ w,
+                const double* __restrict__ lph, const int2* __restrict__ run,
+                const double* __restrict__ rad, const double* __restrict__ cor_col,
+                double* __restrict__ lv, double* __restrict__ lw, int jm, int km, int KP, double dr) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
     if (k >= km) return;
     const size_t plane = (size_t)jm * KP, base = (size_t)j * KP + k;
-    int i0, i1;
-    if (!column_run(solid, base, plane, im, i0, i1)) return;
+    const int2 r = run[base];
     const double cor = cor_col[j];
     double L = 0.0, carry = 0.0;     // carry: the adjoint of f_i from the increment of acc_{i+1}
-    for (int i = i1; i >= i0; i--) {
-        const size_t c = base + i * plane;
-        L += lph[c];                  // the adjoint of acc_i (acc_{i+1} = acc_i + ...)
-        double lf = carry;
-        carry = 0.0;
-        if (i > i0) {
-            lf += 0.5 * dr * L;
-            carry = 0.5 * dr * L;
+    for (int h = r.y; h >= r.x; h -= AH) {
+        double pv[AH], vv[AH], ww[AH], av[AH], aw[AH], rr[AH], lf[AH];
+#pragma unroll
+        for (int u = 0; u < AH; u++) {
+            const int i = max(h - u, r.x);
+            const size_t c = base + i * plane;
+            pv[u] = lph[c];
+            vv[u] = v[c];
+            ww[u] = w[c];
+            av[u] = lv[c];
+            aw[u] = lw[c];
+            rr[u] = rad[i];
         }
-        lv[c] += lf * 2.0 * v[c] / rad[i];
-        lw[c] += lf * (2.0 * w[c] / rad[i] + cor);
+#pragma unroll
+        for (int u = 0; u < AH; u++) {
+            L += pv[u];                   // the adjoint of acc_i (acc_{i+1} = acc_i + ...)
+            lf[u] = carry;
+            carry = 0.0;
+            if (h - u > r.x) {
+                lf[u] += 0.5 * dr * L;
+                carry = 0.5 * dr * L;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < AH; u++) {
+            av[u] += lf[u] * 2.0 * vv[u] / rr[u];
+            aw[u] += lf[u] * (2.0 * ww[u] / rr[u] + cor);
+        }
+#pragma unroll
+        for (int u = 0; u < AH; u++)
+            if (h - u >= r.x) {
+                const size_t c = base + (h - u) * plane;
+                lv[c] = av[u];
+                lw[c] = aw[u];
+            }
     }
 }
 
@@ -749,6 +796,25 @@ int atjup_gpu_rk4_adjoint(AtjupCtx* c, double* const a[4]) {
 
 namespace atjup {
 
+// dst[f] = src[f] for n whole fields in the padded layout, on the context's stream
+int launch_copy_fields(AtjupCtx* c, double* const* dst, const double* const* src, int n) {
+    bool wide = n <= COPY_MAX;
+    for (int f = 0; f < n; f++)
+        wide = wide && !((reinterpret_cast<uintptr_t>(dst[f]) | reinterpret_cast<uintptr_t>(src[f])) % 16);
+    if (!wide) {
+        for (int f = 0; f < n; f++)
+            ATJUP_CUDA(cudaMemcpyAsync(dst[f], src[f], sizeof(double) * c->NP, cudaMemcpyDeviceToDevice,
+                                       c->stream));
+        return ATJUP_OK;
+    }
+    CopyArgs a{};
+    for (int f = 0; f < n; f++) { a.dst[f] = dst[f]; a.src[f] = src[f]; }
+    copy_kernel<<<dim3((unsigned)((c->NP / 4 + 255) / 256), n), 256, 0, c->stream>>>(a, c->NP);
+    c->launches++;
+    ATJUP_CHECK_LAUNCH("copy_fields");
+    return ATJUP_OK;
+}
+
 int rk4_tlm_ext(AtjupCtx* c, double* const d[4], const double* dp, const double* drho,
                 double* const daux[3]) {
     Lin L;
@@ -809,8 +875,7 @@ int rk4_adjoint_ext(AtjupCtx* c, double* const a[4], double* lp, double* lrho,
     const LinConst q = lin_const(c);
     const size_t bytes = sizeof(double) * c->NP;
     // the adjoint of the result, kept: every stage reads it; a[] accumulates the adjoint of Y
-    for (int f = 0; f < 4; f++)
-        ATJUP_CUDA(cudaMemcpyAsync(L.B[f], a[f], bytes, cudaMemcpyDeviceToDevice, c->stream));
+    if ((rc = launch_copy_fields(c, L.B, a, 4))) return rc;
     double* W = L.lv;
     double* lb = L.lv + P.im;
     ATJUP_CUDA(cudaMemsetAsync(L.ph, 0, bytes, c->stream));
@@ -818,7 +883,7 @@ int rk4_adjoint_ext(AtjupCtx* c, double* const a[4], double* lp, double* lrho,
     const dim3 grid((P.km + 127) / 128, P.jm, P.im);
     const unsigned nblk = (unsigned)((c->NP + 255) / 256);
     // stage 3 scatters into A[1]; every later stage's target was cleared by the stage before it
-    for (int f = 0; f < 4; f++) ATJUP_CUDA(cudaMemsetAsync(L.A[1][f], 0, bytes, c->stream));
+    ATJUP_CUDA(cudaMemsetAsync(L.A[1][0], 0, 4 * bytes, c->stream));      // the four are adjacent
     for (int s = 3; s >= 0; s--) {
         double* const* cur = L.A[s & 1];
         double* const* nxt = L.A[(s + 1) & 1];
@@ -843,12 +908,14 @@ int rk4_adjoint_ext(AtjupCtx* c, double* const a[4], double* lp, double* lrho,
         ATJUP_CHECK_LAUNCH("rk4_adjoint: stage");
     }
     // the adjoint of stage 0's input, which is Y itself
-    for (int f = 0; f < 4; f++) add_kernel<<<nblk, 256, 0, c->stream>>>(a[f], L.A[0][f], c->NP);
-    c->launches += 4;
+    AddArgs add{};
+    for (int f = 0; f < 4; f++) { add.y[f] = a[f]; add.x[f] = L.A[0][f]; }
+    add_kernel<<<dim3(nblk, 4), 256, 0, c->stream>>>(add, c->NP);
+    c->launches++;
     // the column integral onto v, w and the level mean onto t
-    ad_hydro_kernel<<<dim3((P.km + 127) / 128, P.jm), 128, 0, c->stream>>>(
-        c->f[ATJUP_F_V], c->f[ATJUP_F_W], L.ph, c->solid, c->rad, c->cor_col, a[2], a[3], P.im,
-        P.jm, P.km, c->KP, P.dr);
+    ad_hydro_kernel<<<dim3((P.km + 63) / 64, P.jm), 64, 0, c->stream>>>(
+        c->f[ATJUP_F_V], c->f[ATJUP_F_W], L.ph, c->run, c->rad, c->cor_col, a[2], a[3], P.jm, P.km,
+        c->KP, P.dr);
     lin_level_partial<<<dim3(LB_PARTS, P.im), LB_THREADS, 0, c->stream>>>(
         c->f[ATJUP_F_T], nullptr, c->f[ATJUP_F_P_STAT], c->solid, c->sin_the, L.part, P.jm, P.km,
         c->KP, q.g, q.rR, q.t_ref);

@@ -217,6 +217,7 @@ int launch_pressure_fold(AtjupCtx* c, double* p);
 int launch_bc(AtjupCtx* c, int which);
 int launch_bc_ptrs(AtjupCtx* c, int which, double* t, double* u, double* v, double* w,
                    double* p_dyn, double* p_stat, bool phys);
+int launch_copy_fields(AtjupCtx* c, double* const* dst, const double* const* src, int n);
 int rk4_tlm_ext(AtjupCtx* c, double* const d[4], const double* dp, const double* drho,
                 double* const daux[3]);
 // stages: the forward's stage inputs X1, X2, X3 of t, u, v, w (12 buffers, stage-major), or null

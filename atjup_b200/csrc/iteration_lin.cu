@@ -476,10 +476,22 @@ __device__ __forceinline__ double fweight(int m, int d, const FQ& q) {
     return ad == 0 ? 1.0 : 0.0;
 }
 
-__global__ void shapiro_i_T_kernel(const double* __restrict__ src, double* __restrict__ dst,
-                                   const int32_t* __restrict__ topo, FQ q) {
+// The filter's transposes take three fields per launch (blockIdx.z = field, level). A cell whose
+// stencils lie wholly in the fluid (hi_j, hi_k of two columns cover the four cells on each side) has
+// the 4th-order weights without a test of its neighbours' floors.
+struct TFields {
+    const double* src[3];
+    double* dst[3];
+};
+#define T_FIELD                                                                                  \
+    const int f_ = blockIdx.z / q.im, i = blockIdx.z - f_ * q.im;                                  \
+    const double* __restrict__ src = f_ == 0 ? F.src[0] : f_ == 1 ? F.src[1] : F.src[2];           \
+    double* __restrict__ dst = f_ == 0 ? F.dst[0] : f_ == 1 ? F.dst[1] : F.dst[2];
+
+__global__ void shapiro_i_T_kernel(TFields F, const int32_t* __restrict__ topo, FQ q) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, i = blockIdx.z;
+    const int j = blockIdx.y;
+    T_FIELD
     if (k >= q.km) return;
     const size_t plane = (size_t)q.jm * q.KP;
     const size_t c = (size_t)i * plane + (size_t)j * q.KP + k;
@@ -506,13 +518,22 @@ __device__ __forceinline__ int out_mode(const bool* f, int o) {
     return (f[x - 2] && f[x + 2]) ? 4 : 2;
 }
 
-__global__ void shapiro_j_T_kernel(const double* __restrict__ src, double* __restrict__ dst,
-                                   const int32_t* __restrict__ topo, FQ q) {
+__global__ void shapiro_j_T_kernel(TFields F, const int32_t* __restrict__ topo,
+                                   const int32_t* __restrict__ hi_j, FQ q) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, i = blockIdx.z;
+    const int j = blockIdx.y;
+    T_FIELD
     if (k >= q.km) return;
     const size_t row = q.KP;
     const size_t c = ((size_t)i * q.jm + j) * row + k;
+    if (j >= 4 && j < q.jm - 4 &&
+        (!q.use_topo || (i >= hi_j[(j - 2) * row + k] && i >= hi_j[(j + 2) * row + k]))) {
+        double acc = 0.0;
+#pragma unroll
+        for (int d = -2; d <= 2; d++) acc += fweight(4, d, q) * src[c - (ptrdiff_t)d * (ptrdiff_t)row];
+        dst[c] = acc;
+        return;
+    }
     bool f[9];
 #pragma unroll
     for (int e = 0; e < 9; e++) {
@@ -531,15 +552,27 @@ __global__ void shapiro_j_T_kernel(const double* __restrict__ src, double* __res
 }
 
 // the k pass on the ring of km-1 meridians; its output km-1 is the copy of output 0
-__global__ void shapiro_k_T_kernel(const double* __restrict__ src, double* __restrict__ dst,
-                                   const int32_t* __restrict__ topo, FQ q) {
+__global__ void shapiro_k_T_kernel(TFields F, const int32_t* __restrict__ topo,
+                                   const int32_t* __restrict__ hi_k, FQ q) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, i = blockIdx.z;
+    const int j = blockIdx.y;
+    T_FIELD
     if (k >= q.km) return;
     const size_t b = ((size_t)i * q.jm + j) * q.KP;
     if (k == q.km - 1) { dst[b + k] = 0.0; return; }   // the seam input is never read
     const int n = q.km - 1;
     auto ring = [n](int kk) { return kk < 0 ? kk + n : (kk >= n ? kk - n : kk); };
+    const int32_t* hr = hi_k + (size_t)j * q.KP;
+    if (!q.use_topo || (i >= hr[ring(k - 2)] && i >= hr[ring(k + 2)])) {
+        double acc = 0.0;
+#pragma unroll
+        for (int d = -2; d <= 2; d++) {
+            const int o = ring(k - d);
+            acc += fweight(4, d, q) * (src[b + o] + (o == 0 ? src[b + q.km - 1] : 0.0));
+        }
+        dst[b + k] = acc;
+        return;
+    }
     bool f[9];
 #pragma unroll
     for (int e = 0; e < 9; e++) f[e] = i >= floor_at(topo, q.use_topo, j, ring(k + e - 4), q.km);
@@ -580,6 +613,7 @@ __global__ void vbal_row_T_kernel(const double* __restrict__ lv, const int32_t* 
     for (int k = threadIdx.x; k < km; k += blockDim.x) {
         if (topo[(size_t)j * km + k] != 0) continue;
         if (k < km - 1) n++;
+#pragma unroll 8
         for (int i = 0; i < im; i++) s += lv[(size_t)i * plane + (size_t)j * KP + k];
     }
     __shared__ double sh[8];
@@ -599,14 +633,18 @@ __global__ void vbal_row_T_kernel(const double* __restrict__ lv, const int32_t* 
     }
 }
 
+// the levels' weights are formed once per block (a division each), not once per cell
 __global__ void vbal_sub_T_kernel(double* __restrict__ lv, const int32_t* __restrict__ topo,
                                   const double* __restrict__ rs, const double* __restrict__ rad,
                                   int im, int jm, int km, int KP, double dr, int zonal) {
+    extern __shared__ double wgt[];
+    for (int i = threadIdx.x; i < im; i += blockDim.x)
+        wgt[i] = vbal_weight(rad, i, im, dr, vbal_I0(rad, im, dr));
+    __syncthreads();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y + 1;
     if (k >= km || topo[(size_t)j * km + k] != 0) return;
     const size_t plane = (size_t)jm * KP, b = (size_t)j * KP + k;
-    const double I0 = vbal_I0(rad, im, dr);
     double S;
     if (zonal) {
         if (k >= km - 1 || rs[2 * j + 1] <= 0.0) return;    // not among the meridians averaged
@@ -615,7 +653,8 @@ __global__ void vbal_sub_T_kernel(double* __restrict__ lv, const int32_t* __rest
         S = 0.0;
         for (int i = 0; i < im; i++) S += lv[b + (size_t)i * plane];
     }
-    for (int i = 0; i < im; i++) lv[b + (size_t)i * plane] -= S * vbal_weight(rad, i, im, dr, I0);
+#pragma unroll 8
+    for (int i = 0; i < im; i++) lv[b + (size_t)i * plane] -= S * wgt[i];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -640,12 +679,14 @@ const int kBaseIds[5] = {ATJUP_F_P_DYN, ATJUP_F_AUX_U, ATJUP_F_AUX_V, ATJUP_F_AU
                          ATJUP_F_RHO_MIX};
 
 int save_base(AtjupCtx* c, const Scratch& S, bool restore) {
+    double* dst[5];
+    const double* src[5];
     for (int f = 0; f < 5; f++) {
         double* live = c->f[kBaseIds[f]];
-        ATJUP_CUDA(cudaMemcpyAsync(restore ? live : S.base[f], restore ? S.base[f] : live,
-                                   sizeof(double) * c->NP, cudaMemcpyDeviceToDevice, c->stream));
+        dst[f] = restore ? live : S.base[f];
+        src[f] = restore ? S.base[f] : live;
     }
-    return ATJUP_OK;
+    return launch_copy_fields(c, dst, src, 5);
 }
 
 int check_supported(AtjupCtx* c, const char* who, int iter_n) {
@@ -799,14 +840,25 @@ int bc_T(AtjupCtx* c, double* const a[LN]) {
     return ATJUP_OK;
 }
 
-int shapiro_T(AtjupCtx* c, double* f) {
+int shapiro_T(AtjupCtx* c, double* const f[3]) {
     const AtjupParams& P = c->P;
     const FQ q = filt_q(c);
-    const dim3 grid((P.km + 127) / 128, P.jm, P.im);
+    const dim3 grid((P.km + 127) / 128, P.jm, P.im * 3);
+    const int32_t *hk = c->floor_hi, *hj = c->floor_hi + (size_t)P.jm * c->KP;
+    // scratch: the RK step's own stage buffers, rewritten by the next step
+    TFields A{}, B{}, C{};
+    for (int x = 0; x < 3; x++) {
+        A.src[x] = f[x];
+        A.dst[x] = c->X1[x];
+        B.src[x] = c->X1[x];
+        B.dst[x] = c->X2[x];
+        C.src[x] = c->X2[x];
+        C.dst[x] = f[x];
+    }
     for (int p = 0; p < P.shapiro_inloop; p++) {
-        shapiro_i_T_kernel<<<grid, 128, 0, c->stream>>>(f, c->tmp, c->topo, q);
-        shapiro_j_T_kernel<<<grid, 128, 0, c->stream>>>(c->tmp, c->tmp2, c->topo, q);
-        shapiro_k_T_kernel<<<grid, 128, 0, c->stream>>>(c->tmp2, f, c->topo, q);
+        shapiro_i_T_kernel<<<grid, 128, 0, c->stream>>>(A, c->topo, q);
+        shapiro_j_T_kernel<<<grid, 128, 0, c->stream>>>(B, c->topo, hj, q);
+        shapiro_k_T_kernel<<<grid, 128, 0, c->stream>>>(C, c->topo, hk, q);
         c->launches += 3;
     }
     ATJUP_CHECK_LAUNCH("iteration adjoint: Shapiro filter");
@@ -820,7 +872,7 @@ int balance_T(AtjupCtx* c, double* lv) {
                                                           c->KP);
         c->launches++;
     }
-    vbal_sub_T_kernel<<<dim3((P.km + 127) / 128, P.jm - 2), 128, 0, c->stream>>>(
+    vbal_sub_T_kernel<<<dim3((P.km + 127) / 128, P.jm - 2), 128, sizeof(double) * P.im, c->stream>>>(
         lv, c->topo, c->dvc, c->rad, P.im, P.jm, P.km, c->KP, P.dr, P.v_massbal_zonal);
     c->launches++;
     ATJUP_CHECK_LAUNCH("iteration adjoint: column balance");
@@ -890,10 +942,7 @@ static int iteration_adjoint_impl(AtjupCtx* c, int32_t iter_n, int32_t first, in
     if ((parts & ATJUP_LIN_BALANCE) && P.v_massbal_stride > 0 && iter_n % P.v_massbal_stride == 0 &&
         (rc = balance_T(c, a[LV])))
         return rc;
-    if ((parts & ATJUP_LIN_SHAPIRO) && P.shapiro_inloop > 0) {
-        for (int f = LU; f <= LW; f++)
-            if ((rc = shapiro_T(c, a[f]))) return rc;
-    }
+    if ((parts & ATJUP_LIN_SHAPIRO) && P.shapiro_inloop > 0 && (rc = shapiro_T(c, a + LU))) return rc;
     if ((parts & ATJUP_LIN_BC) && (rc = bc_T(c, a))) return rc;
     if (parts & ATJUP_LIN_RK4) {
         double* a4[4] = {a[LT], a[LU], a[LV], a[LW]};

@@ -697,13 +697,16 @@ hydrostatic_kernel(const double* __restrict__ v, const double* __restrict__ w,
             pb[u] = p_baro ? p_baro[c] : 0.0;
             rr[u] = rad[i];
         }
+        double f[HY_AHEAD];               // the divisions are independent: only the sum is a chain
+#pragma unroll
+        for (int u = 0; u < HY_AHEAD; u++)
+            f[u] = 0.0 + ((vv[u] * vv[u] + ww[u] * ww[u]) / rr[u] + cor * ww[u]) / 1.0;
 #pragma unroll
         for (int u = 0; u < HY_AHEAD; u++) {
             const int i = h + u;
             if (i > r.y) break;
-            const double f = 0.0 + ((vv[u] * vv[u] + ww[u] * ww[u]) / rr[u] + cor * ww[u]) / 1.0;
-            if (i > r.x) acc = acc + 0.5 * (fprev + f) * dr;
-            fprev = f;
+            if (i > r.x) acc = acc + 0.5 * (fprev + f[u]) * dr;
+            fprev = f[u];
             ph[base + i * plane] = acc + pb[u];
         }
     }

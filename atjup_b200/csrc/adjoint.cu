@@ -20,6 +20,7 @@
 // The stencils, the solid-face mirroring of p_hydro, the ring in phi and the integrated-cell mask
 // are those of the forward kernel (rk4.cu), so the two directions are transposes of each other.
 #include "ctx.cuh"
+#include "quot.cuh"
 
 namespace atjup {
 namespace {
@@ -660,8 +661,15 @@ ad_hydro_kernel(const double* __restrict__ v, const double* __restrict__ w,
         }
 #pragma unroll
         for (int u = 0; u < AH; u++) {
-            av[u] += lf[u] * 2.0 * vv[u] / rr[u];
-            aw[u] += lf[u] * (2.0 * ww[u] / rr[u] + cor);
+            const double x = lf[u] * 2.0 * vv[u], y = 2.0 * ww[u];
+            if (quot_ok(x, rr[u]) && quot_ok(y, rr[u])) {
+                const double ir = rcp_of(rr[u]);
+                av[u] += quot(x, rr[u], ir);
+                aw[u] += lf[u] * (quot(y, rr[u], ir) + cor);
+            } else {
+                av[u] += x / rr[u];
+                aw[u] += lf[u] * (y / rr[u] + cor);
+            }
         }
 #pragma unroll
         for (int u = 0; u < AH; u++)

@@ -20,6 +20,7 @@
 // cells) keep their live values through the step: stages 0-2 copy the live field into the next
 // stage input there, as the reference's untouched live arrays do.
 #include "ctx.cuh"
+#include "quot.cuh"
 
 namespace atjup {
 namespace {
@@ -160,7 +161,7 @@ __device__ __forceinline__ int precip_slot(int s) {
 template <typename R>
 struct CellShared {
     R u0, v_invrm, w_invrs, two_inv_rm, inv_rm2, ci, is2, nue_t_s;
-    double rho;
+    R fall;                    // the NH4SH crystals' fall speed over u_0
 };
 
 // The right-hand side of species S at a cell from its stencil and sources
@@ -185,9 +186,7 @@ __device__ __forceinline__ R species_rhs(const PhysStage& a, const CellShared<R>
         r = -transport + diffusion * coef + (R)(a.chemical_reaction * src0) +
             (R)(a.precip_coupling * src1);
     } else if constexpr (S == ATJUP_S_NH4SH) {
-        const double v_stokes = a.stokes_pre * (a.rg_nh4sh - z.rho) * a.g / a.mue_mix;
-        r = -transport + (R)src0 + diffusion * coef + (R)(a.chemical_reaction * src1) +
-            (R)(v_stokes / a.u_0) * d1r;
+        r = -transport + (R)src0 + diffusion * coef + (R)(a.chemical_reaction * src1) + z.fall * d1r;
     } else {
         r = -transport + diffusion * coef + (R)(a.precip_coupling * src0);
     }
@@ -314,9 +313,20 @@ __global__ void __launch_bounds__(256, 3) species_stage_kernel(PhysStage a) {
     z.is2 = (R)g.inv_rm2sinthe2;
     double nue_t64 = 0.0;
     if (a.has_nue && a.turb_coupling != 0.0 && isfinite(nv)) nue_t64 = a.turb_coupling * dmax(0.0, nv);
-    const R nue_t = (R)nue_t64;
-    z.nue_t_s = nue_t / (R)0.9;
-    z.rho = rho;
+    // nue_t / 0.9 and the crystals' fall speed over u_0 (the NH4SH species' own), each by its constant
+    // divisor's reciprocal (quot.cuh)
+    if constexpr (sizeof(R) == 8) {
+        const double n[2] = {nue_t64, a.stokes_pre * (a.rg_nh4sh - rho) * a.g}, d[2] = {0.9, a.mue_mix};
+        double o[2], f[1];
+        quots(n, d, o);
+        z.nue_t_s = (R)o[0];
+        const double n2[1] = {o[1]}, d2[1] = {a.u_0};
+        quots(n2, d2, f);
+        z.fall = (R)f[0];
+    } else {
+        z.nue_t_s = (R)nue_t64 / (R)0.9;
+        z.fall = (R)(a.stokes_pre * (a.rg_nh4sh - rho) * a.g / a.mue_mix / a.u_0);
+    }
     species_all<0, TI, TO, TA, R>(a, x, z, species_load<0, TI, TA, R>(a, x));
 }
 
@@ -417,7 +427,26 @@ __global__ void __launch_bounds__(256, 3) closure_stage_kernel(PhysStage a) {
     const R dtkedthe_s = dtkedthe * inv_rm, ddisdthe_s = ddisdthe * inv_rm;
     const R dtkedphi_s = dtkedphi * inv_rmsinthe, ddisdphi_s = ddisdphi * inv_rmsinthe;
     const R grad_dot = dtkedr * ddisdr + dtkedthe_s * ddisdthe_s + dtkedphi_s * ddisdphi_s;
-    R cnue = (MODEL == ATJUP_TURB_K_EPSILON) ? C_nue * tke_s * tke_s / dis_s : tke_s / dis_s;
+    const double y_mount = layer_h(a, topo) * 1.0e3;
+    const double dz_layer = dmax(1.0, layer_dz_m(a, i - 1 > 0 ? i - 1 : 0));
+    const double y_phys = dmax(layer_h(a, i) * 1.0e3 - y_mount, dz_layer);
+    // The cell's quotients in groups (quot.cuh): one after another their divisions were most of the
+    // kernel's latency. Here those of the closure's own values: the eddy viscosity's ratio, y / L, and
+    // the SST model's 2 sig_w2 / omega.
+    R cnue, y_star, sst_r = (R)0;
+    {
+        const R num = (MODEL == ATJUP_TURB_K_EPSILON) ? C_nue * tke_s * tke_s : tke_s;
+        if constexpr (sizeof(R) == 8) {
+            const R n[3] = {num, (R)y_phys, (R)2 * (R)1.168}, d[3] = {dis_s, (R)L_m, dis_s};
+            R o[3];
+            quots(n, d, o);
+            cnue = o[0]; y_star = o[1]; sst_r = o[2];
+        } else {
+            cnue = num / dis_s;
+            y_star = (R)(y_phys / L_m);
+            sst_r = (R)2 * (R)1.168 / dis_s;
+        }
+    }
     cnue = dmin(cnue, (R)a.nue_max);
     const R c23 = (R)0.66667, two = (R)2;
     const R der = c23 * (dudr_s + dvdthe_s + dwdphi_s);
@@ -432,29 +461,37 @@ __global__ void __launch_bounds__(256, 3) closure_stage_kernel(PhysStage a) {
         + (cnue * (dwdr_s + dudphi_s)) * dwdr_s
         + (cnue * (dwdthe_s + dvdphi_s)) * dwdthe_s);
 
-    const double y_mount = layer_h(a, topo) * 1.0e3;
-    const double dz_layer = dmax(1.0, layer_dz_m(a, i - 1 > 0 ? i - 1 : 0));
-    const double y_phys = dmax(layer_h(a, i) * 1.0e3 - y_mount, dz_layer);
-    const R y_star = (R)(y_phys / L_m);
     const R inv_re = (R)a.inv_re;
 
     R dtre, ddre, tke_src, dis_src, c_w_prod;
     if (MODEL == ATJUP_TURB_K_EPSILON) {                      // Chien 1982
         const R sig_k = (R)1.0, sig_w = (R)1.3, C_eps_1 = (R)1.35, C_eps_2 = (R)1.80;
-        dtre = inv_re + nue_here / sig_k;
-        ddre = inv_re + nue_here / sig_w;
         // the wall-damping exponentials in FP64: their arguments overflow FP32 near dis_min
-        const double d_plus = y_phys * a.vel_star[(size_t)j * a.KP + k] / nue_gas_phys;
         const double tke_d = (double)tke_s, dis_d = (double)dis_s;
-        const double Re_T = tke_d * tke_d * a.u_0 * L_m / (dis_d * nue_gas_phys);
-        const R f_2 = (R)(1.0 - 0.4 / 1.8 * exp(-Re_T * Re_T / 36.0));
         const R y_star2 = y_star * y_star;
-        const R L_k = -(R)2 * tk0 / y_star2;
-        const R L_w = (R)(-2.0 * (double)ds0 / (double)y_star2 * exp(-0.5 * d_plus));
-        const R P_w = C_eps_1 * ds0 / tke_s * P_full;
-        const R Y_w = C_eps_2 * f_2 * ds0 * ds0 / tke_s;
-        tke_src = P_full - ds0 + L_k / (R)a.re_turb;
-        dis_src = P_w - Y_w + L_w / (R)a.re_turb;
+        double w[3];
+        {
+            const double n[3] = {y_phys * a.vel_star[(size_t)j * a.KP + k], tke_d * tke_d * a.u_0 * L_m,
+                                 -2.0 * (double)ds0};
+            const double d[3] = {nue_gas_phys, dis_d * nue_gas_phys, (double)y_star2};
+            quots(n, d, w);
+        }
+        const double d_plus = w[0], Re_T = w[1];
+        const R f_2 = (R)(1.0 - 0.4 / 1.8 * exp(-Re_T * Re_T / 36.0));
+        const R L_w = (R)(w[2] * exp(-0.5 * d_plus));
+        const R n[5] = {nue_here, nue_here, -(R)2 * tk0, C_eps_1 * ds0, C_eps_2 * f_2 * ds0 * ds0};
+        const R d[5] = {sig_k, sig_w, y_star2, tke_s, tke_s};
+        R o[5];
+        quots(n, d, o);
+        dtre = inv_re + o[0];
+        ddre = inv_re + o[1];
+        const R P_w = o[3] * P_full;
+        const R Y_w = o[4];
+        const R nl[2] = {o[2], L_w}, dl[2] = {(R)a.re_turb, (R)a.re_turb};
+        R ol[2];
+        quots(nl, dl, ol);
+        tke_src = P_full - ds0 + ol[0];
+        dis_src = P_w - Y_w + ol[1];
         c_w_prod = C_eps_1;
     } else if (MODEL == ATJUP_TURB_K_OMEGA) {                 // Wilcox
         const R sig_k = (R)0.6, sig_w = (R)0.5, bet_star = (R)0.09, gam = (R)0.52;
@@ -473,15 +510,27 @@ __global__ void __launch_bounds__(256, 3) closure_stage_kernel(PhysStage a) {
         const R Omega = sqrt(W12 * W12 + W13 * W13 + W23 * W23);
         // the vortex-stretching ratio in FP64: (0.09 omega*)^3 underflows FP32 near dis_min
         const double bd = 0.09 * (double)dis_s;
-        const double chi_w = fabs((double)Omega * (double)Omega * (double)S_mag / (bd * bd * bd));
-        const double f_bet = (1.0 + 85.0 * chi_w) / (1.0 + 100.0 * chi_w);
+        double o1[1], o2[1];
+        {
+            const double n[1] = {(double)Omega * (double)Omega * (double)S_mag}, d[1] = {bd * bd * bd};
+            quots(n, d, o1);
+        }
+        const double chi_w = fabs(o1[0]);
+        {
+            const double n[1] = {1.0 + 85.0 * chi_w}, d[1] = {1.0 + 100.0 * chi_w};
+            quots(n, d, o2);
+        }
+        const double f_bet = o2[0];
         const R bet_wc = (R)(bet_0 * f_bet);
         const R sig_d = (grad_dot <= (R)0) ? (R)0 : (R)0.125;
         const R P_k = dmin(P_full, (R)20 * bet_star * tke_s * dis_s);
         const R Y_k = bet_star * tke_s * dis_s;
-        const R P_w = gam * dis_s / tke_s * P_k;
+        const R n[2] = {gam * dis_s, sig_d}, d[2] = {tke_s, dis_s};
+        R o[2];
+        quots(n, d, o);
+        const R P_w = o[0] * P_k;
         const R Y_w = bet_wc * dis_s * dis_s;
-        const R D_w = sig_d / dis_s * grad_dot;
+        const R D_w = o[1] * grad_dot;
         tke_src = P_k - Y_k;
         dis_src = P_w - Y_w + D_w;
         c_w_prod = gam;
@@ -490,22 +539,32 @@ __global__ void __launch_bounds__(256, 3) closure_stage_kernel(PhysStage a) {
         const R sig_w2 = (R)1.168;
         const R bet1 = (R)0.0333, bet2 = (R)0.0368, gam1 = (R)0.413, gam2 = (R)0.2;
         const R nue_air_nd = (R)(nue_gas_phys / (a.u_0 * L_m));
-        const R CD_kw = dmax((R)2 * sig_w2 / dis_s * grad_dot, (R)1.0e-20);
-        const R arg1 = dmin(dmax(sqrt(dmax(tk0, (R)0)) / (bet_star * dis_s * y_star),
-                                 (R)500 * nue_air_nd / (y_star * y_star * dis_s)),
-                            (R)4 * sig_w2 * tke_s / (CD_kw * y_star * y_star));
+        const R CD_kw = dmax(sst_r * grad_dot, (R)1.0e-20);
+        R arg1;
+        {
+            const R n[3] = {sqrt(dmax(tk0, (R)0)), (R)500 * nue_air_nd, (R)4 * sig_w2 * tke_s};
+            const R d[3] = {bet_star * dis_s * y_star, y_star * y_star * dis_s, CD_kw * y_star * y_star};
+            R o[3];
+            quots(n, d, o);
+            arg1 = dmin(dmax(o[0], o[1]), o[2]);
+        }
         const R a2 = arg1 * arg1;
         const R F1 = tanh(a2 * a2);                                          // pow(arg1, 4)
         const R one = (R)1;
         const R sig_k = F1 * sig_k1 + (one - F1) * sig_k2;
         const R sig_w = F1 * sig_w1 + (one - F1) * sig_w2;
-        dtre = inv_re + nue_here / sig_k;
-        ddre = inv_re + nue_here / sig_w;
         const R P_k = dmin(P_full, (R)20 * bet_star * tke_s * dis_s);
         const R Y_k = bet_star * tke_s * dis_s;
-        const R P_w = (F1 * gam1 + (one - F1) * gam2) * P_k * dis_s / tke_s;
+        const R n[4] = {nue_here, nue_here, (F1 * gam1 + (one - F1) * gam2) * P_k * dis_s,
+                        (R)2 * (one - F1) * sig_w2};
+        const R d[4] = {sig_k, sig_w, tke_s, dis_s};
+        R o[4];
+        quots(n, d, o);
+        dtre = inv_re + o[0];
+        ddre = inv_re + o[1];
+        const R P_w = o[2];
         const R Y_w = (F1 * bet1 + (one - F1) * bet2) * dis_s * dis_s;
-        const R D_w = (R)2 * (one - F1) * sig_w2 / dis_s * grad_dot;
+        const R D_w = o[3] * grad_dot;
         tke_src = P_k - Y_k;
         dis_src = P_w - Y_w + D_w;
         c_w_prod = F1 * gam1 + (one - F1) * gam2;

@@ -12,6 +12,7 @@
 // marches a tile of columns up through the radial planes; each plane's inputs reach shared memory
 // two planes ahead as tensor-memory-accelerator copies (cp.async.bulk.tensor on mbarriers).
 #include "ctx.cuh"
+#include "quot.cuh"
 
 #include <cuda.h>
 
@@ -448,10 +449,11 @@ rk_stage_kernel(StagePtrs a, StageConst q, const __grid_constant__ StageMaps M) 
 
                 // compression work with the hydrostatic part (RHS_Jup_Turb.cpp:459-482)
                 const double rho_l = S.ex[xs][0][tid];
+                const bool rho_ok = rho_l > 0.0 && isfinite(rho_l);
                 double dpstatdr64 = 0.0;
                 if (q.adiabatic) {
                     dpstatdr64 = (S.ps[ns][tid] - m_ps) * q.inv_2dr * q.to_nd;
-                    if (q.adiabatic_rho && rho_l > 0.0 && isfinite(rho_l)) dpstatdr64 *= q.r_mix / rho_l;
+                    if (q.adiabatic_rho && rho_ok) dpstatdr64 *= quot1(q.r_mix, rho_l);
                 }
                 const R dpstatdr = (R)dpstatdr64;
                 const R pressure_t = (R)q.coeff_energy_p *
@@ -500,25 +502,24 @@ rk_stage_kernel(StagePtrs a, StageConst q, const __grid_constant__ StageMaps M) 
                 double radiation_t = 0.0, precip_t = 0.0;
                 if (q.has_heating) {
                     if (q.rad_coupling != 0.0) {
-                        const double T_phys = (double)t0 * q.t_ref;
-                        const double P_phys = S.ps[cs][tid] * 1.0e5;
-                        const double rho = (rho_l > 0.0 && isfinite(rho_l))
-                                               ? rho_l
-                                               : ((T_phys > 1.0) ? P_phys / (q.R_mix * T_phys) : 0.0);
+                        double rho = rho_l;
+                        if (!rho_ok) {
+                            const double T_phys = (double)t0 * q.t_ref, P_phys = S.ps[cs][tid] * 1.0e5;
+                            rho = (T_phys > 1.0) ? P_phys / (q.R_mix * T_phys) : 0.0;
+                        }
                         if (rho > 0.0 && q.cp_mix > 0.0) {
-                            radiation_t = q.rad_coupling * S.ex[xs][3][tid] * q.L_rad /
-                                          (rho * q.cp_mix * q.u_0 * q.t_ref);
+                            radiation_t = quot1(q.rad_coupling * S.ex[xs][3][tid] * q.L_rad,
+                                                rho * q.cp_mix * q.u_0 * q.t_ref);
                             if (!isfinite(radiation_t)) radiation_t = 0.0;
                             else if (radiation_t > 0.5) radiation_t = 0.5;
                             else if (radiation_t < -0.5) radiation_t = -0.5;
                         }
                     }
                     if (q.precip_coupling != 0.0) {
-                        double rho_p = q.r_mix;
-                        if (q.precip_local) rho_p = (rho_l > 0.0 && isfinite(rho_l)) ? rho_l : q.r_mix;
+                        const double rho_p = (q.precip_local && rho_ok) ? rho_l : q.r_mix;
                         if (rho_p > 0.0 && q.cp_mix > 0.0) {
-                            precip_t = q.precip_coupling * S.ex[xs][4][tid] * q.L_rad /
-                                       (rho_p * q.cp_mix * q.u_0 * q.t_ref);
+                            precip_t = quot1(q.precip_coupling * S.ex[xs][4][tid] * q.L_rad,
+                                             rho_p * q.cp_mix * q.u_0 * q.t_ref);
                             if (!isfinite(precip_t)) precip_t = 0.0;
                             else if (precip_t > 0.5) precip_t = 0.5;
                             else if (precip_t < -0.5) precip_t = -0.5;
@@ -526,12 +527,12 @@ rk_stage_kernel(StagePtrs a, StageConst q, const __grid_constant__ StageMaps M) 
                     }
                 }
 
-                double nue_t = 0.0;
+                double nue_t = 0.0, nue_t_s = 0.0;
                 if (q.has_nue) {
                     const double nn = S.ex[xs][2][tid];
                     if (q.turb_coupling != 0.0 && isfinite(nn)) nue_t = q.turb_coupling * fmax(0.0, nn);
+                    nue_t_s = quot_ok(nue_t, 0.9) ? quot(nue_t, 0.9, 1.0 / 0.9) : nue_t / 0.9;
                 }
-                const double nue_t_s = nue_t / 0.9;
                 const R visc = (R)(q.inv_re + nue_t + S.ex[xs][1][tid]);
 
                 const R rhs_t = +pressure_t - transport_t + diffusion_t * (R)(q.t_visc + nue_t_s) +
@@ -539,7 +540,7 @@ rk_stage_kernel(StagePtrs a, StageConst q, const __grid_constant__ StageMaps M) 
                 // the buoyancy anomaly against the level mean, in FP64 (the mean is FP64)
                 const double t0d = (double)t0;
                 const double buoyancy_u =
-                    (t0d > 0.0) ? q.buoy_k * (q.g * S.ps[cs][tid] / (q.rR * t0d * q.t_ref) - a.buoy_ref[i])
+                    (t0d > 0.0) ? q.buoy_k * (quot1(q.g * S.ps[cs][tid], q.rR * t0d * q.t_ref) - a.buoy_ref[i])
                                 : 0.0;
                 const R rhs_u = -dpdr_term + (q.hydro_split ? (R)0.0 : (R)buoyancy_u) - transport_u +
                                 diffusion_u * visc - (R)(q.cor_rad_on * q.Coriolis) * Coriolis_rad +
@@ -630,12 +631,25 @@ buoy_partial_kernel(const double* __restrict__ t, const double* __restrict__ p_s
             pv[u] = p_stat[c];
             wv[u] = sin_the[on[u] ? j : 0];
         }
+        double bv[BR_AHEAD];
+        bool ok = true;
 #pragma unroll
         for (int u = 0; u < BR_AHEAD; u++) {
-            if (!on[u] || !(tv[u] > 0.0)) continue;
-            const double bb = g * pv[u] / (rR * tv[u] * t_ref);
-            if (!isfinite(bb)) continue;
-            s += wv[u] * bb;
+            on[u] = on[u] && tv[u] > 0.0;
+            if (!on[u]) { tv[u] = 1.0; pv[u] = 0.0; }
+            ok = ok && quot_ok(g * pv[u], rR * tv[u] * t_ref);
+        }
+        if (ok) {
+#pragma unroll
+            for (int u = 0; u < BR_AHEAD; u++)
+                bv[u] = quot(g * pv[u], rR * tv[u] * t_ref, rcp_of(rR * tv[u] * t_ref));
+        } else {
+            for (int u = 0; u < BR_AHEAD; u++) bv[u] = g * pv[u] / (rR * tv[u] * t_ref);
+        }
+#pragma unroll
+        for (int u = 0; u < BR_AHEAD; u++) {
+            if (!on[u] || !isfinite(bv[u])) continue;
+            s += wv[u] * bv[u];
             ws += wv[u];
         }
     }
@@ -697,10 +711,21 @@ hydrostatic_kernel(const double* __restrict__ v, const double* __restrict__ w,
             pb[u] = p_baro ? p_baro[c] : 0.0;
             rr[u] = rad[i];
         }
-        double f[HY_AHEAD];               // the divisions are independent: only the sum is a chain
+        double f[HY_AHEAD], e[HY_AHEAD];
+        bool ok = true;
 #pragma unroll
-        for (int u = 0; u < HY_AHEAD; u++)
-            f[u] = 0.0 + ((vv[u] * vv[u] + ww[u] * ww[u]) / rr[u] + cor * ww[u]) / 1.0;
+        for (int u = 0; u < HY_AHEAD; u++) {
+            e[u] = vv[u] * vv[u] + ww[u] * ww[u];
+            ok = ok && quot_ok(e[u], rr[u]);
+        }
+        if (ok) {
+#pragma unroll
+            for (int u = 0; u < HY_AHEAD; u++) e[u] = quot(e[u], rr[u], rcp_of(rr[u]));
+        } else {
+            for (int u = 0; u < HY_AHEAD; u++) e[u] = e[u] / rr[u];
+        }
+#pragma unroll
+        for (int u = 0; u < HY_AHEAD; u++) f[u] = 0.0 + (e[u] + cor * ww[u]) / 1.0;
 #pragma unroll
         for (int u = 0; u < HY_AHEAD; u++) {
             const int i = h + u;

@@ -27,6 +27,7 @@
 // the file is compiled without FMA contraction; the parcel test compares a virtual-temperature
 // difference with 1e-7 K, so a last-bit difference of exp/log can flip a marginal pair.
 #include "ctx.cuh"
+#include "quot.cuh"
 
 namespace atjup {
 namespace {
@@ -54,6 +55,9 @@ struct McaArgs {
     double tr_ep[NT], tr_L[NT];
     int tr_cond[NT];
     double cp, grav, t_ref, r_mix, relax;
+    double cp_r;                       // 1 / cp
+    double kR[NG], kR_r[NG];           // 1e-3 R of the gases' vapour-pressure fits, and 1 / that
+    double iep[NG], tr_iep[NT];        // 1 / ep - 1
     int im, jm, km, KP, local_rho, ledoux, loading, max_pass;
     unsigned long long* stats;         // [8], then NPART pairs of census partial counts
     unsigned* colflag;                 // [jm * km]
@@ -62,64 +66,94 @@ struct McaArgs {
     uint8_t* pairs;                    // [im * jm * km] census of pair (i, i+1): bit 0 unstable, bit 1 moist
 };
 
-// ATPhys.h:49-52 [bar], with log(T) passed in: both gases are evaluated at the same T, and the
-// logarithm (a pure function) is the same value whether computed once or per gas
-__device__ __forceinline__ double svp(double T, double lT, double C, double L0, double R, double da,
-                                      double db) {
-    return exp(C + (-L0 / T + da * lT + db * T) / (1e-3 * R));
-}
-// the phase's coefficients are selected first, so the saturation curve is one exp in the code
-// (the liquid and ice curves are the same expression on different constants)
-__device__ __forceinline__ double qsat(const McaArgs& a, int g, double T, double lT, double p) {
-    const AtjupGasParams& s = a.gas[g];
-    const bool liq = T >= s.t_0;
-    const double E = svp(T, lT, liq ? s.C : s.C_i, liq ? s.L0 : s.L0_i, s.R,
-                         liq ? s.del_alf : s.del_alf_i, liq ? s.del_bet : s.del_bet_i);
-    const double q = s.ep * E / p;
-    return isfinite(q) ? q : 0.0;
+// q_sat of both gases at (T, p), pr = rcp_of(p) (ATPhys.h:49-52 [bar]). Both are evaluated at the same T,
+// so the logarithm and the reciprocal of T are shared; the phase's coefficients are selected first, so a
+// saturation curve is one exp in the code (the liquid and ice curves are the same expression on
+// different constants). The six divisions of the reference's expressions are quotients by T, by the
+// constant 1e-3 R and by p, formed side by side (quot.cuh): one after another they were most of a solve.
+__device__ __forceinline__ void qsat2(const McaArgs& a, double T, double p, double pr, double (&q)[NG]) {
+    const double lT = log(T);
+    double n[NG], x[NG], E[NG];
+#pragma unroll
+    for (int g = 0; g < NG; g++) n[g] = -(T >= a.gas[g].t_0 ? a.gas[g].L0 : a.gas[g].L0_i);
+    quots_by(n, T, rcp_of(T), x);
+#pragma unroll
+    for (int g = 0; g < NG; g++) {
+        const AtjupGasParams& s = a.gas[g];
+        const bool liq = T >= s.t_0;
+        n[g] = x[g] + (liq ? s.del_alf : s.del_alf_i) * lT + (liq ? s.del_bet : s.del_bet_i) * T;
+    }
+    quots(n, a.kR, a.kR_r, x);
+#pragma unroll
+    for (int g = 0; g < NG; g++) {
+        const AtjupGasParams& s = a.gas[g];
+        E[g] = exp((T >= s.t_0 ? s.C : s.C_i) + x[g]);
+        n[g] = s.ep * E[g];
+    }
+    quots_by(n, p, pr, q);
+#pragma unroll
+    for (int g = 0; g < NG; g++) q[g] = isfinite(q[g]) ? q[g] : 0.0;
 }
 __device__ __forceinline__ double lat(const McaArgs& a, int g, double T) {
     return T >= a.gas[g].t_0 ? a.gas[g].lv : a.gas[g].ls;
 }
-__device__ __forceinline__ double fof(const McaArgs& a, double TT, double hL, const double* qt,
-                                      double p, double z) {
-    double f = a.cp * TT + a.grav * z - hL;
-    const double lT = log(TT);
-    for (int g = 0; g < NG; g++) f -= lat(a, g, TT) * dmax(0.0, qt[g] - qsat(a, g, TT, lT, p));
-    return f;
+// the bracket's ends: all vapour, and the rise with all of q_t condensed
+__device__ __forceinline__ double all_vapour(const McaArgs& a, double hL, double z) {
+    return quot1_by(hL - a.grav * z, a.cp, a.cp_r);
 }
-// equilibrium temperature of (h_L, q_t) at (p, z): Illinois regula falsi in [all vapour, all
-// condensed] (ConvectiveAdjustment.h:459-486)
-__device__ bool equil(const McaArgs& a, double hL, const double* qt, double p, double z, double& T,
-                      double* cond) {
-    const double T_lo = (hL - a.grav * z) / a.cp;
-    if (!(T_lo > 0.0) || !(p > 0.0)) return false;
-    bool any = false;
-    const double lT_lo = log(T_lo);
-    for (int g = 0; g < NG; g++)
-        if (qt[g] > qsat(a, g, T_lo, lT_lo, p)) { any = true; break; }
-    if (!any) {
-        T = T_lo;
-        for (int g = 0; g < NG; g++) cond[g] = 0.0;
-        return true;
-    }
+__device__ __forceinline__ double all_condensed(const McaArgs& a, double T_lo, const double* qt) {
     double span = 0.0;
     for (int g = 0; g < NG; g++) span += dmax(a.gas[g].lv, a.gas[g].ls) * dmax(0.0, qt[g]);
-    double lo = T_lo, hi = T_lo + span / a.cp + 1.0e-9;
-    double flo = fof(a, lo, hL, qt, p, z), fhi = fof(a, hi, hL, qt, p, z);
+    return T_lo + quot1_by(span, a.cp, a.cp_r) + 1.0e-9;
+}
+// equilibrium temperature of (h_L, q_t) at (p, z): Illinois regula falsi in [all vapour, all
+// condensed] (ConvectiveAdjustment.h:459-486). One place evaluates the balance, for the bracket's ends
+// as for the iterates: inlined at each of the reference's five, and again for each solve of a pair, the
+// code outgrew the instruction cache (half of the census kernel's stalls). The condensate at the
+// solution is that of the last evaluation there (the solution is always a point that was evaluated).
+__device__ __forceinline__ bool equil(const McaArgs& a, double hL, const double* qt, double p, double z, double& T,
+                                      double* cond) {
+    const double T_lo = all_vapour(a, hL, z);
+    if (!(T_lo > 0.0) || !(p > 0.0)) return false;
+    const double pr = rcp_of(p);
+    double x = T_lo, lo = T_lo, hi = T_lo, flo = 0.0, fhi = 0.0;
     int side = 0;
-    for (int it = 0; it < NITER && hi - lo > TOL_T; it++) {
-        double c = (fhi - flo != 0.0) ? hi - fhi * (hi - lo) / (fhi - flo) : 0.5 * (lo + hi);
-        if (!(c > lo && c < hi)) c = 0.5 * (lo + hi);
-        const double fc = fof(a, c, hL, qt, p, z);
-        if (fc < 0.0) { lo = c; flo = fc; if (side == -1) fhi *= 0.5; side = -1; }
-        else          { hi = c; fhi = fc; if (side == +1) flo *= 0.5; side = +1; }
-        if (fabs(fc) <= a.cp * TOL_T) { lo = hi = c; break; }
+    // step -2 at T_lo, -1 at the warm end, then the iterates
+#pragma unroll 1
+    for (int it = -2;; it++) {
+        double qs[NG], ex[NG];
+        qsat2(a, x, p, pr, qs);
+        double f = a.cp * x + a.grav * z - hL;
+        bool any = false;
+#pragma unroll
+        for (int g = 0; g < NG; g++) {
+            any = any || qt[g] > qs[g];
+            ex[g] = dmax(0.0, qt[g] - qs[g]);
+            f -= lat(a, g, x) * ex[g];
+        }
+        bool done = false;
+        if (it == -2) {
+            flo = f;
+            if (any) hi = all_condensed(a, T_lo, qt);
+            else { ex[0] = ex[1] = 0.0; done = true; }
+        } else if (it == -1) {
+            fhi = f;
+        } else {
+            if (f < 0.0) { lo = x; flo = f; if (side == -1) fhi *= 0.5; side = -1; }
+            else         { hi = x; fhi = f; if (side == +1) flo *= 0.5; side = +1; }
+            if (fabs(f) <= a.cp * TOL_T) { hi = x; done = true; }
+        }
+        if (x == hi) {
+            T = x;
+#pragma unroll
+            for (int g = 0; g < NG; g++) cond[g] = ex[g];
+        }
+        if (done) return true;
+        if (it == -2) { x = hi; continue; }
+        if (!(it + 1 < NITER && hi - lo > TOL_T)) return true;
+        x = (fhi - flo != 0.0) ? hi - quot1(fhi * (hi - lo), fhi - flo) : 0.5 * (lo + hi);
+        if (!(x > lo && x < hi)) x = 0.5 * (lo + hi);
     }
-    T = hi;
-    const double lT = log(T);
-    for (int g = 0; g < NG; g++) cond[g] = dmax(0.0, qt[g] - qsat(a, g, T, lT, p));
-    return true;
 }
 
 // One cell's conserved state: mass fractions, h_L, and the inputs of the parcel test.
@@ -137,15 +171,25 @@ __device__ bool load_cell(const McaArgs& a, int i, size_t c, Cell& x) {
     x.rho = r;
     if (!(x.T > 0.0) || !(x.p > 0.0) || !(x.rho > 0.0) || !isfinite(x.T + x.p + x.rho)) return false;
     double h = a.cp * x.T + a.grav * x.z;
+    double n[3 * NG + NT], q[3 * NG + NT];
+#pragma unroll
     for (int g = 0; g < NG; g++) {
-        x.qv[g] = dmax(0.0, a.vap[g][c]) / x.rho;
-        x.qc[g] = dmax(0.0, a.cld[g][c]) / x.rho;
-        x.qi[g] = dmax(0.0, a.ice[g][c]) / x.rho;
+        n[3 * g] = dmax(0.0, a.vap[g][c]);
+        n[3 * g + 1] = dmax(0.0, a.cld[g][c]);
+        n[3 * g + 2] = dmax(0.0, a.ice[g][c]);
+    }
+#pragma unroll
+    for (int r2 = 0; r2 < NT; r2++) n[3 * NG + r2] = a.trf[r2][c];
+    quots_by(n, x.rho, rcp_of(x.rho), q);
+#pragma unroll
+    for (int g = 0; g < NG; g++) {
+        x.qv[g] = q[3 * g]; x.qc[g] = q[3 * g + 1]; x.qi[g] = q[3 * g + 2];
         x.qt[g] = x.qv[g] + x.qc[g] + x.qi[g];
         h -= a.gas[g].lv * x.qc[g] + a.gas[g].ls * x.qi[g];
     }
+#pragma unroll
     for (int r2 = 0; r2 < NT; r2++) {
-        x.qr[r2] = a.trf[r2][c] / x.rho;
+        x.qr[r2] = q[3 * NG + r2];
         h -= a.tr_L[r2] * x.qr[r2];
     }
     x.hL = h;
@@ -161,23 +205,62 @@ __device__ __forceinline__ double tv(const McaArgs& a, double TT, const double* 
     if (!a.ledoux) return TT;
     double f = 1.0;
     for (int g = 0; g < NG; g++) {
-        f += v[g] * (1.0 / a.gas[g].ep - 1.0);
+        f += v[g] * a.iep[g];
         if (a.loading) f -= cnd[g];
     }
     for (int r = 0; r < NT; r++) {
         const double q = qr[r];
-        if (a.tr_ep[r] > 0.0) f += q * (1.0 / a.tr_ep[r] - 1.0);
+        if (a.tr_ep[r] > 0.0) f += q * a.tr_iep[r];
         else if (a.tr_cond[r] && a.loading) f -= q;
     }
     return TT * f;
 }
-// the parcel test of a below b (ConvectiveAdjustment.h:651-665) given b's own equilibrium
-__device__ bool pair_test(const McaArgs& a, double hLa, const double* qta, const double* qra,
-                          double pb, double zb, double Tb, const double* ecb, const double* qtb,
-                          const double* qrb, bool& ok, bool* held, bool* moist) {
-    double Tp, pc[NG], pv[NG], ev[NG];
-    ok = equil(a, hLa + trE(a, qra), qta, pb, zb, Tp, pc);
-    if (!ok) return false;
+// A level's temperature and virtual temperature over every state its solve can end in: T in its bracket
+// [T0, T1] (all vapour, all condensed), each condensate in [0, q_t]. False where the bounds do not hold (a
+// solve that is refused, a factor that is not positive, a T so large that rounding could reach the test's
+// 1e-7 K, a NaN).
+struct Range { double T0, T1, v0, v1; };
+__device__ __forceinline__ bool tv_range(const McaArgs& a, double hL, double z, const double* qt, const double* qr,
+                                         Range& R) {
+    double f0 = 1.0, f1 = 1.0;
+    if (a.ledoux) {
+#pragma unroll
+        for (int g = 0; g < NG; g++) {
+            const double dry = qt[g] * a.iep[g], wet = a.loading ? -qt[g] : 0.0;
+            f0 += dry < wet ? dry : wet;
+            f1 += dry < wet ? wet : dry;
+        }
+#pragma unroll
+        for (int r = 0; r < NT; r++) {
+            double x = 0.0;
+            if (a.tr_ep[r] > 0.0) x = qr[r] * a.tr_iep[r];
+            else if (a.tr_cond[r] && a.loading) x = -qr[r];
+            f0 += x;
+            f1 += x;
+        }
+    }
+    R.T0 = all_vapour(a, hL, z);
+    R.T1 = all_condensed(a, R.T0, qt);
+    R.v0 = R.T0 * f0;
+    R.v1 = R.T1 * f1;
+    return R.T0 > 0.0 && f0 > 0.0 && f1 < 10.0 && R.T1 < 1.0e5;
+}
+// What the ranges of the parcel lifted from lo and of the air at up settle: a parcel that is at its lightest no
+// lighter than the air at its heaviest is not unstable, whatever the solves would add.
+// 0 undecided, 1 stable, 2 held by composition (the census counts those).
+__device__ __forceinline__ int settled(const McaArgs& a, const Cell& lo, const Cell& up) {
+    Range P, B;
+    if (!tv_range(a, lo.hL + trE(a, lo.qr), up.z, lo.qt, lo.qr, P) ||
+        !tv_range(a, up.hL + trE(a, up.qr), up.z, up.qt, up.qr, B) || !(P.v1 <= B.v0))
+        return 0;
+    return P.T1 <= B.T0 ? 1 : (P.T0 - B.T1 > 2.0 * TOL_K ? 2 : 0);
+}
+// the parcel test of a below b (ConvectiveAdjustment.h:651-665) given the parcel's equilibrium (Tp, pc) and
+// b's own (Tb, ecb)
+__device__ __forceinline__ bool pair_compare(const McaArgs& a, double Tp, const double* pc, const double* qta,
+                                             const double* qra, double Tb, const double* ecb, const double* qtb,
+                                             const double* qrb, bool* held, bool* moist) {
+    double pv[NG], ev[NG];
     bool wet = false;
     for (int g = 0; g < NG; g++) {
         pv[g] = qta[g] - pc[g];
@@ -210,7 +293,10 @@ __global__ void mca_bounds_kernel(const uint8_t* solid, int2* bounds, int im, in
 
 // one thread per pair (i, i+1): the census of the unadjusted column. Capped at 64 registers
 // (eight blocks per SM): the solve is a chain of dependent FP64 exp/log, and the extra warps hide
-// more of it than the few spilled values cost.
+// more of it than the spilled values cost (4, 6 and 8 blocks: 426, 366 and 348 us on the 41x181x361
+// shell; 646 us with the compiler's divisions and a balance inlined per evaluation). Bound by
+// instruction issue. A pair takes about 18 evaluations of the balance unless settled() spares them, a
+// third of the pairs there (394 us without it).
 __global__ void __launch_bounds__(128, 8) mca_census_kernel(McaArgs a) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
     unsigned long long ut = 0, hd = 0;
@@ -224,10 +310,25 @@ __global__ void __launch_bounds__(128, 8) mca_census_kernel(McaArgs a) {
             if (!v0 || !v1) {
                 enqueue(a, col);       // the column thread counts it as skipped
             } else {
-                double Tb, ecb[NG];
-                bool ok = equil(a, up.hL + trE(a, up.qr), up.qt, up.p, up.z, Tb, ecb);
-                bool held = false, moist = false, uns = false;
-                if (ok) uns = pair_test(a, lo.hL, lo.qt, lo.qr, up.p, up.z, Tb, ecb, up.qt, up.qr, ok, &held, &moist);
+                bool moist = false, uns = false;
+                const int st = settled(a, lo, up);
+                bool held = st == 2;
+                if (st == 0) {
+                    // the air at i+1, then the parcel from i there: one solve in the code
+                    double Tb = 0.0, Tp = 0.0, ecb[NG] = {0.0, 0.0}, pc[NG] = {0.0, 0.0};
+                    bool ok = true;
+#pragma unroll 1
+                    for (int s = 0; s < 2 && ok; s++) {
+                        double qt[NG];
+                        for (int g = 0; g < NG; g++) {
+                            ecb[g] = pc[g];
+                            qt[g] = s ? lo.qt[g] : up.qt[g];
+                        }
+                        Tb = Tp;
+                        ok = equil(a, s ? lo.hL + trE(a, lo.qr) : up.hL + trE(a, up.qr), qt, up.p, up.z, Tp, pc);
+                    }
+                    if (ok) uns = pair_compare(a, Tp, pc, lo.qt, lo.qr, Tb, ecb, up.qt, up.qr, &held, &moist);
+                }
                 if (uns || held) ut = 1;
                 if (held) hd = 1;
                 a.pairs[((size_t)i * a.jm + j) * a.km + k] = (uint8_t)((uns ? 1 : 0) | (moist ? 2 : 0));
@@ -263,15 +364,20 @@ struct Col {
 };
 
 __device__ bool col_unstable(const McaArgs& a, Col& C, int lo, int up, bool* held, bool* moist) {
-    if (!C.eq_ok[up]) {
-        if (!equil(a, C.hL[up] + trE(a, C.qr[up]), C.qt[up], C.p[up], C.z[up], C.Teq[up], C.ceq[up]))
-            return false;
-        C.eq_ok[up] = 1;
+    // the air's solve unless it is cached, then the parcel's: one solve in the code (the reference solves
+    // the parcel before the cached air state; both are pure functions)
+    double Tp, pc[NG];
+#pragma unroll 1
+    for (int s = C.eq_ok[up] ? 1 : 0; s < 2; s++) {
+        const int q = s ? lo : up;
+        if (!equil(a, C.hL[q] + trE(a, C.qr[q]), C.qt[q], C.p[up], C.z[up], Tp, pc)) return false;
+        if (s == 0) {
+            C.Teq[up] = Tp;
+            for (int g = 0; g < NG; g++) C.ceq[up][g] = pc[g];
+            C.eq_ok[up] = 1;
+        }
     }
-    // the reference solves the parcel before the cached air state; both are pure functions
-    bool ok;
-    return pair_test(a, C.hL[lo], C.qt[lo], C.qr[lo], C.p[up], C.z[up], C.Teq[up], C.ceq[up],
-                     C.qt[up], C.qr[up], ok, held, moist);
+    return pair_compare(a, Tp, pc, C.qt[lo], C.qr[lo], C.Teq[up], C.ceq[up], C.qt[up], C.qr[up], held, moist);
 }
 __device__ bool col_settle(const McaArgs& a, Col& C, int q) {
     double TT, pc[NG];
@@ -660,6 +766,13 @@ int launch_mca(AtjupCtx* c) {
     a.tr_ep[0] = M.ep_h2s; a.tr_cond[0] = 0; a.tr_L[0] = 0.0;
     a.tr_ep[1] = 0.0;      a.tr_cond[1] = 1; a.tr_L[1] = M.L_nh4sh;
     a.cp = P.cp_mix;
+    a.cp_r = 1.0 / a.cp;
+    for (int g = 0; g < NG; g++) {
+        a.kR[g] = 1e-3 * a.gas[g].R;
+        a.kR_r[g] = 1.0 / a.kR[g];
+        a.iep[g] = 1.0 / a.gas[g].ep - 1.0;
+    }
+    for (int r = 0; r < NT; r++) a.tr_iep[r] = 1.0 / a.tr_ep[r] - 1.0;   // read only where ep > 0
     a.grav = P.g;
     a.t_ref = P.t_ref;
     a.r_mix = P.r_mix;

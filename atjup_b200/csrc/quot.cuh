@@ -60,6 +60,37 @@ __device__ __forceinline__ void quots(const double (&a)[N], const double (&b)[N]
         for (int q = 0; q < N; q++) o[q] = a[q] / b[q];
     }
 }
+// o[q] = a[q] / b with r = rcp_of(b) (or the host's 1.0 / b, the same bits): a divisor used many times
+template <int N>
+__device__ __forceinline__ void quots_by(const double (&a)[N], double b, double r, double (&o)[N]) {
+    bool ok = true;
+#pragma unroll
+    for (int q = 0; q < N; q++) ok = ok && quot_ok(a[q], b);
+    if (ok) {
+#pragma unroll
+        for (int q = 0; q < N; q++) o[q] = quot(a[q], b, r);
+    } else {
+#pragma unroll
+        for (int q = 0; q < N; q++) o[q] = a[q] / b;
+    }
+}
+// o[q] = a[q] / b[q] with r[q] = rcp_of(b[q])
+template <int N>
+__device__ __forceinline__ void quots(const double (&a)[N], const double (&b)[N], const double (&r)[N], double (&o)[N]) {
+    bool ok = true;
+#pragma unroll
+    for (int q = 0; q < N; q++) ok = ok && quot_ok(a[q], b[q]);
+    if (ok) {
+#pragma unroll
+        for (int q = 0; q < N; q++) o[q] = quot(a[q], b[q], r[q]);
+    } else {
+#pragma unroll
+        for (int q = 0; q < N; q++) o[q] = a[q] / b[q];
+    }
+}
+__device__ __forceinline__ double quot1_by(double a, double b, double r) {
+    return quot_ok(a, b) ? quot(a, b, r) : a / b;
+}
 // FP32 divisions overlap as they are
 template <int N>
 __device__ __forceinline__ void quots(const float (&a)[N], const float (&b)[N], float (&o)[N]) {

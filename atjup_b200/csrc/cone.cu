@@ -25,25 +25,31 @@
 //
 // Each level is one thread-block cluster of C blocks (C = 4, or fewer when the GPU cannot hold
 // every level's cluster at once: 26 levels on 104 SMs for the 41 x 181 x 361 grid). Block r owns
-// a band of the box's rows with its phi, cell flags and per-cell constants in shared memory; the
-// rows next to its band are read from the neighbouring blocks' shared memory (distributed shared
-// memory), and a cluster barrier ends each step. Each sweep's largest change and largest |phi|
-// are kept per block in a ring slot (the band's first cell of the sweep opens it, the other cells
-// raise it by a shared-memory atomic maximum on the IEEE bit pattern, issued only when a cell
-// exceeds the value it reads); sweep t is complete after step D + 2(t-1) (D = NJ + NK - 2), where
-// every block reads the C slots and takes the stopping test. The sweeps after the converged one
-// have by then already updated the first diagonals; each block restores its band from the newest
-// snapshot that precedes them (one every SNAP_EVERY steps, in HBM) and the cluster replays up to
-// the converged sweep. The arithmetic is the reference's, operation for operation (this file is
-// compiled without FMA contraction), so the result is the reference's to the bit.
+// a band of the box's rows with its phi, cell flags and constants in shared memory, and copies of the
+// rows next to its band: the block that updates an edge row stores the new values in the neighbour's
+// copy too (distributed shared memory), so every load is a local one. Each sweep's largest change and
+// largest |phi| are kept per block in a ring slot; sweep t is complete after step D + 2(t-1)
+// (D = NJ + NK - 2). Every CHECK_STEPS steps the blocks take the stopping test of the sweeps completed
+// since, reading the C slots of each. The sweeps after the converged one have by then already updated
+// the first diagonals; each block restores its band from the newest snapshot that precedes them (one
+// every SNAP_EVERY steps, in HBM) and the cluster replays up to the converged sweep. The arithmetic is
+// the reference's, operation for operation (this file is compiled without FMA contraction but for the
+// quotients, which equal the division), so the result is the reference's to the bit.
+//
+// What bounds it: the issue of a step's instructions and its chain of dependent FP64 operations, on few
+// cells (1500 a block and step on the 41 x 181 x 361 grid); no memory traffic to speak of. One projection
+// there takes 5.7 ms (12.7 ms with the cells over all warps, the compiler's division, every cell
+// raising its sweep's slot and a cluster barrier each step), 61 x 97 2.5 ms (4.9), 33 x 41 1.0 ms (1.6).
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include <cooperative_groups.h>
 
 #include "ctx.cuh"
+#include "quot.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -55,10 +61,13 @@ constexpr double CONE_OMEGA = 1.9;       // InitValues_Jup.cpp:1726
 constexpr int CONE_MAXIT = 40000;        // InitValues_Jup.cpp:1728
 constexpr double CONE_TOL = 1.0e-10;     // InitValues_Jup.cpp:1761
 constexpr int SNAP_EVERY = 64;           // wavefront steps between snapshots
-constexpr int CONE_THREADS = 1024;
 constexpr int CONE_CLUSTER = 4;          // blocks per level (fewer when the GPU cannot hold them)
 constexpr size_t CONE_SMEM_CAP = 200 * 1024;
-constexpr int NROW = 6;                  // per box row: aN, aS, aL, s, s dphi, A of a plain cell
+constexpr int CHECK_STEPS = 16;          // wavefront steps between stopping tests
+// per box row: aN, aS, aL, A of a plain cell, 1 / A, s, s dphi (and one unused: rows of 64 bytes, read
+// two doubles at a time)
+constexpr int NROW = 8;
+enum { RC_N, RC_S, RC_L, RC_A, RC_RA, RC_SJ, RC_SD };
 
 // cell flags of the box (uint32 per cell: these bits, the special-cell index above bit 6)
 enum : uint32_t { CF_SOLID = 1, CF_N = 2, CF_S = 4, CF_W = 8, CF_E = 16, CF_NEAR = 32 };
@@ -70,12 +79,12 @@ constexpr uint32_t CF_WALL = CF_N | CF_S | CF_W | CF_E;
 // 0..NJ+1, b' = b + 1 in 0..NK+1) sits at ((c (NJ + 2) + a') PW + b' / 2), c = (a' + b') mod 2;
 // the flags of interior cell (a, b) at ((c NJ + a) PW + (b + 1) / 2).
 struct ConeLevel {
-    int i, jlo, klo, NJ, NK, PW, D, n_spec;
+    int i, jlo, klo, NJ, NK, PW, D, n_spec, n_tab;
     int64_t info_off;   // uint32 [2 * NJ * PW]: flags | special index << 6
     int64_t spec_off;   // int32 [n_spec]: (c NJ + a) PW + m of each special cell
     int64_t phi_off;    // double [2 * (NJ + 2) * PW] per warm-start buffer (halo included)
-    int64_t snap_off;   // double [n_snap * C * 2 * (nbmax + 2) * PW]: per block, its band
-    int64_t tab_off;    // double [2 * n_spec] (global-memory mode)
+    int64_t snap_off;   // double [n_snap * C * 2 * (nbmax + 2) * PW]: per block, its band and the rows beside it
+    int64_t tab_off;    // double [n_tab] (global-memory mode)
     int64_t row_off;    // double [NROW * NJ] (global-memory mode)
     int n_snap, ring;
 };
@@ -95,6 +104,8 @@ struct ConeState {
     int C = 1;                              // blocks (one cluster) per level
     int ring_max = 1;                       // the largest ring of the levels
     bool smem_mode = true;
+    const void* kernel = nullptr;           // the form of cone_kernel for the levels' bands, and its threads
+    int threads = 0;
     size_t smem = 0;                        // dynamic shared memory per block
     int64_t n_phi = 0;
 };
@@ -117,130 +128,310 @@ struct ConeArgs {
     double* w;
     const uint8_t* solid;
     const double* rad;
-    int jm, km, KP, H, smem_mode, C, ring_max;
+    int jm, km, KP, H, C, ring_max;
     double dr, dthe, dphi;
 };
 
 // A block's band of a level's box as the kernel sees it. Local row la = 1..nb is box row
 // a = A0 + la - 1 (halo coordinate a' = A0 + la); the words of colour x, local row la start at
-// phi + x cs + la PW, la = 0 and nb + 1 being the rows beside the band (nrow, srow per colour:
-// the neighbouring block's rows in its shared memory, or the box's halo).
+// phi + x cs + la PW, la = 0 and nb + 1 being the copies of the rows beside the band (or the box's halo).
 struct Box {
     double* phi;
     int cs;                     // colour stride of phi
-    const double* nrow[2];
-    const double* srow[2];
     const uint32_t* info;       // flags of local row la, colour x at info + x ics + (la - 1) PW
     int ics;
     const double* tab;
-    const double* rows;         // [NROW][NJ], indexed by box row
+    const double* rows;         // [NJ][NROW], indexed by box row
     unsigned long long* ring;   // [2 R]: largest change, largest |phi| of sweep t at t mod R
+    double *push_n, *push_s;    // the neighbours' copies of this band's first and last row (colour 0), or null
+    unsigned bar_n, bar_s;      // RowForm: those copies' barriers there, and this block's own (shared addresses)
+    unsigned bar;
     int NJ, NK, PW, D, R;       // R a power of two
-    int lgCH;                   // the row's words of one colour in 2^lgCH chunks of 32
     int nb, A0;
     bool div;
+    bool recip;                 // every row's A has a reciprocal quot() takes
     double dthe, dphi;
 };
 
-__device__ __forceinline__ const double* row_of(const Box& B, int x, int la) {
-    if (la == 0) return B.nrow[x];
-    if (la == B.nb + 1) return B.srow[x];
-    return B.phi + x * B.cs + la * B.PW;
-}
-
 // phi of the cell at local row la (0..nb+1), halo column b' (0..NK+1)
 __device__ __forceinline__ double phi_at(const Box& B, int la, int bp) {
-    return row_of(B, (B.A0 + la + bp) & 1, la)[bp >> 1];
-}
-
-// One SOR update of the cell at local row la, colour c, word m (InitValues_Jup.cpp:1739-1758), in
-// the reference's order of operations. Returns false for a cell the sweep skips (solid, or no
-// fluid face: A = 0); else the change and |phi| in dch, pabs.
-__device__ __forceinline__ bool cone_update(const Box& B, int la, int c, int m, int off,
-                                            double& dch, double& pabs) {
-    const uint32_t inf = B.info[c * B.ics + (la - 1) * B.PW + m];
-    if (inf & CF_SOLID) return false;
-    const int a = B.A0 + la - 1;
-    const double* rc = B.phi + (c ^ 1) * B.cs + la * B.PW;   // this row, the other colour
-    const double pN = row_of(B, c ^ 1, la - 1)[m], pS = row_of(B, c ^ 1, la + 1)[m];
-    const double pW = rc[m - 1 + off], pE = rc[m + off];
-    const double aN = B.rows[a], aS = B.rows[B.NJ + a], aL = B.rows[2 * B.NJ + a];
-    double A, Bs = 0.0;
-    if (!(inf & (CF_WALL | CF_NEAR)) || (!B.div && !(inf & CF_WALL))) {
-        // a plain cell: all four faces fluid
-        A = B.rows[5 * B.NJ + a];
-        Bs += aN * pN;
-        Bs += aS * pS;
-        Bs += aL * pW;
-        Bs += aL * pE;
-    } else if (B.div && (inf & CF_NEAR)) {
-        A = 0.0;
-        if (!(inf & CF_N)) { A += aN; Bs += aN * pN; }
-        if (!(inf & CF_S)) { A += aS; Bs += aS * pS; }
-        if (!(inf & CF_W)) { A += aL; Bs += aL * pW; }
-        if (!(inf & CF_E)) { A += aL; Bs += aL * pE; }
-        Bs += B.tab[2 * (inf >> 6)];
-    } else {
-        A = 0.0;
-        const double vp = B.tab[2 * (inf >> 6)], wp = B.tab[2 * (inf >> 6) + 1];
-        const double sj = B.rows[3 * B.NJ + a];
-        if (inf & CF_N) Bs -= aN * B.dthe * (-vp); else { A += aN; Bs += aN * pN; }
-        if (inf & CF_S) Bs -= aS * B.dthe * (vp);  else { A += aS; Bs += aS * pS; }
-        if (inf & CF_W) Bs -= aL * sj * B.dphi * (-wp); else { A += aL; Bs += aL * pW; }
-        if (inf & CF_E) Bs -= aL * sj * B.dphi * (wp);  else { A += aL; Bs += aL * pE; }
-    }
-    if (!(A > 0.0)) return false;
-    double* own = B.phi + c * B.cs + la * B.PW + m;
-    const double p = *own;
-    const double pn = p + CONE_OMEGA * (Bs / A - p);
-    dch = fabs(pn - p);
-    *own = pn;
-    pabs = fabs(pn);
-    return true;
+    return B.phi[((B.A0 + la + bp) & 1) * B.cs + la * B.PW + (bp >> 1)];
 }
 
 // std::max(cur, x) as the reference folds it (a NaN x leaves cur), on the ring's bit patterns
-__device__ __forceinline__ void ring_raise(unsigned long long* slot, double x) {
-    if (x > __longlong_as_double((long long)*(volatile unsigned long long*)slot))
-        atomicMax(slot, (unsigned long long)__double_as_longlong(x));
+__device__ __forceinline__ void ring_raise(unsigned long long* slot, double cur, double x) {
+    if (x > cur) atomicMax(slot, (unsigned long long)__double_as_longlong(x));
 }
 
-// One cell of a wavefront step tau on the block's band: the cell of colour tau mod 2 at local row
-// la, word m, if its sweep t = (tau - a - b) / 2 + 1 lies in [1, t_stop].
-__device__ __forceinline__ void cone_cell(const Box& B, int tau, int t_stop, bool reduce, int la,
-                                          int m) {
-    const int c = tau & 1;
-    const int a = B.A0 + la - 1;
-    const int off = (c ^ (a + 1)) & 1;              // b' of word 0 of this colour in row a'
-    const int b = off + 2 * m - 1;
-    if (b < 0 || b >= B.NK) return;
-    const int diff = tau - a - b;
-    if (diff < 0) return;
-    const int t = (diff >> 1) + 1;
-    if (t > t_stop) return;
-    double dch = 0.0, pabs = 0.0;
-    const bool upd = cone_update(B, la, c, m, off, dch, pabs);
-    if (!reduce) return;
-    unsigned long long* slot = B.ring + 2 * (t & (B.R - 1));
-    if (la == 1 && b == 0) {
-        // the band's first cell of the sweep, alone in its sweep here at this step: opens the
-        // band's slot
-        slot[0] = (unsigned long long)__double_as_longlong(upd && dch > 0.0 ? dch : 0.0);
-        slot[1] = (unsigned long long)__double_as_longlong(upd && pabs > 0.0 ? pabs : 0.0);
-    } else if (upd) {
-        ring_raise(slot, dch);
-        ring_raise(slot + 1, pabs);
+// The constants of a box row: aN, aS, aL, A of a plain cell, rcp_of(A).
+struct RowCoef {
+    double N, S, L, A, rA;
+};
+__device__ __forceinline__ RowCoef row_coef(const Box& B, int la) {
+    const double2* rc = reinterpret_cast<const double2*>(B.rows + (size_t)(B.A0 + la - 1) * NROW);
+    const double2 c0 = rc[0], c1 = rc[1];
+    return RowCoef{c0.x, c0.y, c1.x, c1.y, rc[2].x};
+}
+
+// A special cell's entry in tab, at 2 (f >> 6): of a wall cell A, rcp_of(A), the four faces' prescribed terms (zero
+// in the divergence solve) and the divergence's source; of a cell near the body without a wall the source.
+constexpr int TAB_WALL = 8, TAB_NEAR = 2;
+
+// B and A of a cell with flags f and neighbours pN, pS, pW, pE (InitValues_Jup.cpp:1739-1758), in the reference's
+// order of operations; r = rcp_of(A). (What a wall face adds to B is a constant of the cell.)
+__device__ __forceinline__ double cone_sum(const RowCoef& R, double pN, double pS, double pW, double pE) {
+    double Bs = R.N * pN;
+    Bs += R.S * pS;
+    Bs += R.L * pW;
+    Bs += R.L * pE;
+    return Bs;
+}
+__device__ __forceinline__ double cone_special(const Box& B, const RowCoef& R, uint32_t f, double Bs, double pN, double pS,
+                                               double pW, double pE, double& A, double& r) {
+    const double2* t = reinterpret_cast<const double2*>(B.tab) + (f >> 6);
+    if (!(f & CF_WALL)) return B.div ? Bs + t[0].x : Bs;
+    const double2 a = t[0], k0 = t[1], k1 = t[2];
+    Bs = f & CF_N ? k0.x : R.N * pN;
+    Bs += f & CF_S ? k0.y : R.S * pS;
+    Bs += f & CF_W ? k1.x : R.L * pW;
+    Bs += f & CF_E ? k1.y : R.L * pE;
+    A = a.x;
+    r = a.y;
+    return B.div ? Bs + t[3].x : Bs;
+}
+// quot() takes the sum (A's side is B.recip)
+__device__ __forceinline__ bool sum_ok(double Bs) {
+    return 2u * (unsigned)__double2hiint(Bs) - (623u << 21) < (801u << 21);
+}
+
+// raises the band's slot of the sweep a cell with this diff = tau - a - b is in, or opens it
+__device__ __forceinline__ void raise(const Box& B, unsigned diff, bool opens, double dch, double pabs) {
+    unsigned long long* slot = B.ring + 2 * ((int)((diff >> 1) + 1) & (B.R - 1));
+    if (opens) {
+        slot[0] = (unsigned long long)__double_as_longlong(dch > 0.0 ? dch : 0.0);
+        slot[1] = (unsigned long long)__double_as_longlong(pabs > 0.0 ? pabs : 0.0);
+    } else {
+        const double2 cur = *reinterpret_cast<const double2*>(slot);   // at most as large as it is now
+        ring_raise(slot, cur.x, dch);
+        ring_raise(slot + 1, cur.y, pabs);
     }
 }
 
-// One wavefront step tau on the block's band. Warp w owns chunk w mod 2^lgCH of the local rows
-// 1 + w / 2^lgCH + n 32 / 2^lgCH: lane l updates word 32 chunk + l of each (no division).
-__device__ void cone_step(const Box& B, int tau, int t_stop, bool reduce) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m = ((warp & ((1 << B.lgCH) - 1)) << 5) + lane;
-    const int la_step = (blockDim.x >> 5) >> B.lgCH;
-    for (int la = 1 + (warp >> B.lgCH); la <= B.nb; la += la_step) cone_cell(B, tau, t_stop, reduce, la, m);
+// The block's and the cluster's barriers, for code that a block's warps take in different copies.
+__device__ __forceinline__ void block_sync() { asm volatile("barrier.sync.aligned 0;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+
+// The two forms of a wavefront step tau on the block's band: the cells of colour tau mod 2 whose sweep
+// t = (tau - a - b) / 2 + 1 lies in [1, t_stop]; t2 = 2 t_stop.
+
+// Any band: the 2^lg chunks of 32 words of a row go to neighbouring warps; lane l updates word
+// 32 chunk + l of its rows, and every cell raises the ring slot itself.
+struct WordForm {
+    static constexpr int THREADS = 1024;
+    int m, la0, la_step;
+    __device__ __forceinline__ void init(const Box& B) {
+        const int warp = threadIdx.x >> 5;
+        int lg = 0;
+        while ((32 << lg) < B.PW) lg++;
+        m = ((warp & ((1 << lg) - 1)) << 5) + (threadIdx.x & 31);
+        la0 = 1 + (warp >> lg);
+        la_step = (THREADS / 32) >> lg;
+    }
+    __device__ __forceinline__ void load(const Box&) {}
+    __device__ __forceinline__ bool settle(const Box&) { return true; }
+    __device__ __forceinline__ void end_step() { cluster_sync(); }
+    __device__ static bool odd_row(const Box&) { return false; }
+    template <bool PAR, int c, bool REDUCE>
+    __device__ __forceinline__ void step(const Box& B, int tau, unsigned t2) {
+        for (int la = la0; la <= B.nb; la += la_step) {
+            const int off = (c ^ (B.A0 + la)) & 1;              // b' of word 0 of this colour in the row
+            const int b = off + 2 * m - 1;
+            const unsigned diff = (unsigned)(tau - (B.A0 + la - 1) - b);
+            if ((unsigned)b >= (unsigned)B.NK || diff >= t2) continue;
+            const uint32_t f = B.info[c * B.ics + (la - 1) * B.PW + m];
+            double dch = 0.0, pabs = 0.0;
+            if (!(f & CF_SOLID)) {
+                const int own = c * B.cs + la * B.PW + m;
+                const double* n = B.phi + (c ^ 1) * B.cs + la * B.PW + m;
+                const RowCoef R = row_coef(B, la);
+                const double p = B.phi[own], pN = n[-B.PW], pS = n[B.PW], pW = n[off - 1], pE = n[off];
+                double Bs = cone_sum(R, pN, pS, pW, pE), A = R.A, r = R.rA;
+                if (f) Bs = cone_special(B, R, f, Bs, pN, pS, pW, pE, A, r);
+                if (A > 0.0) {
+                    const double x = B.recip && sum_ok(Bs) ? quot(Bs, A, r) : Bs / A;
+                    const double pn = p + CONE_OMEGA * (x - p);
+                    B.phi[own] = pn;
+                    if (la == 1 && B.push_n) B.push_n[c * B.cs + m] = pn;
+                    if (la == B.nb && B.push_s) B.push_s[c * B.cs + m] = pn;
+                    dch = fabs(pn - p);
+                    pabs = fabs(pn);
+                }
+            }
+            // the band's first cell of the sweep, alone in it here at this step, opens the slot
+            if (REDUCE) raise(B, diff, la == 1 && m == 0, dch, pabs);
+        }
+    }
+};
+
+// Bands of 2 to 28 rows of at most 64 words a colour: a warp per row, a lane with four consecutive cells of it,
+// b = 4 lane - 1 + {0, 1, 2, 3}, of which a step takes the two of its colour: those with even b' (phase 0)
+// or odd b' (phase 1), in turn. The row's constants and the lane's four values stay in registers, so a cell's
+// west and east neighbours are there or one lane away, and a step loads the rows to the north and south, two
+// words each, and stores two.
+//
+// A sweep is in a word at phase 0, again at phase 1, then in the next word. So its largest change and |phi|
+// over the row travel with it from word to word, and at the row's last word they raise the band's ring slot:
+// row la one step after row la - 1, so plain loads and stores do (each cell raising the slot by atomics took more
+// instructions than its update: on 64 bits of shared memory they are loops, and the changes grow along a
+// sweep more often than not).
+//
+// The block's barrier ends a step. Only the warps of the band's edge rows wait for a neighbour: each stores its
+// row there every step with st.async, which counts the bytes on the neighbour's barrier of that side and
+// colour, and waits for the neighbour's row before its own next step (two barriers a side: a row of
+// one colour is sent only after the neighbour's row of the other colour arrived, so a phase is over before the
+// next one's bytes come). A cluster barrier for each step took 725 cycles, more than the step's work.
+struct RowForm {
+    static constexpr int ROWS = 28, THREADS = 32 * ROWS, WORDS = 64;
+    double val[2][2];                    // [phase][word]
+    double md[2], mp[2];                 // largest change and |phi| of the sweep in each word
+    RowCoef R;
+    int start[2][2];                     // the step of a cell's first sweep (never, for a cell the sweeps skip)
+    unsigned special;                    // bit 2 P + w: the cell is a special one
+    int q[2];                            // the lane's two words of each phase, in phi
+    unsigned push, bar_there, bar_here;  // edge rows: the neighbour's copy of them (colour 0), the barriers (colour 0)
+    unsigned phases;                     // parity of each colour's barrier
+    int e0, la, lane, waiting;           // waiting: colour of the neighbour's row not waited for yet, or -1
+    bool row_ok, edge, dead;
+    __device__ __forceinline__ void init(const Box& B) {
+        lane = threadIdx.x & 31;
+        la = 1 + (threadIdx.x >> 5);
+        row_ok = la <= B.nb;
+        if (!row_ok) la = 1;
+        const int m = 2 * lane;
+        const int par = (B.A0 + la) & 1;
+        R = row_coef(B, la);
+        const int m_end = B.NK >> 1;     // the row's last word, at b = 2 m (or past the last cell, b = NK)
+        special = 0;
+        e0 = lane == (m_end >> 1) ? B.A0 + la - 1 + 2 * m_end : INT_MAX;
+#pragma unroll
+        for (int P = 0; P < 2; P++) {
+            const int c = P ^ par;
+            q[P] = c * B.cs + la * WORDS + m;
+#pragma unroll
+            for (int w = 0; w < 2; w++) {
+                const int b = 4 * lane + 2 * w + P - 1;
+                uint32_t x = CF_SOLID;
+                if (row_ok && b >= 0 && b < B.NK) x = B.info[c * B.ics + (la - 1) * WORDS + m + w];
+                const double A = x & CF_WALL ? B.tab[2 * (x >> 6)] : R.A;
+                const bool skip = (x & CF_SOLID) || !(A > 0.0);
+                start[P][w] = skip ? INT_MIN : B.A0 + la - 1 + b;
+                if (!skip && ((x & CF_WALL) || (B.div && (x & CF_NEAR)))) special |= 1u << (2 * P + w);
+            }
+        }
+        md[0] = md[1] = mp[0] = mp[1] = 0.0;
+        double* to = la == 1 ? B.push_n : la == B.nb ? B.push_s : nullptr;      // a band has two rows at least
+        edge = row_ok && to;
+        if (edge) {
+            push = (unsigned)__cvta_generic_to_shared(to) + 8 * m;
+            bar_there = la == 1 ? B.bar_n : B.bar_s;
+            bar_here = B.bar + (la == 1 ? 0 : 16);
+        }
+        waiting = -1;
+        load(B);
+    }
+    __device__ __forceinline__ void load(const Box& B) {
+#pragma unroll
+        for (int P = 0; P < 2; P++) {
+            const double2 x = *reinterpret_cast<const double2*>(B.phi + q[P]);
+            val[P][0] = x.x;
+            val[P][1] = x.y;
+        }
+    }
+    // waits for the neighbour's row of the last step; false (from then on) when it did not come
+    __device__ __forceinline__ bool settle(const Box& B) {
+        if (waiting < 0) return !dead;
+        const unsigned b = bar_here + 8 * waiting, ph = (phases >> waiting) & 1;
+        if (lane == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(b), "r"(8 * WORDS) : "memory");
+        unsigned done = dead;
+        for (int tries = 0; !done && tries < (1 << 16); tries++)
+            asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                         " selp.u32 %0, 1, 0, p;\n}" : "=r"(done) : "r"(b), "r"(ph) : "memory");
+        if (!done) dead = true;
+        phases ^= 1u << waiting;
+        waiting = -1;
+        return !dead;
+    }
+    template <int P, int c, bool REDUCE>
+    __device__ __forceinline__ void phase(const Box& B, int tau, unsigned t2) {
+        if (edge) settle(B);
+        const double2 n = *reinterpret_cast<const double2*>(B.phi + q[1 - P] - WORDS);
+        const double2 s = *reinterpret_cast<const double2*>(B.phi + q[1 - P] + WORDS);
+        const double(&o)[2] = val[1 - P];
+        double W[2], E[2];
+        if (P == 0) {
+            W[0] = __shfl_up_sync(0xffffffffu, o[1], 1); E[0] = o[0];
+            W[1] = o[0]; E[1] = o[1];
+            if (REDUCE) {
+                const double d = __shfl_up_sync(0xffffffffu, md[1], 1), x = __shfl_up_sync(0xffffffffu, mp[1], 1);
+                md[1] = md[0]; mp[1] = mp[0];
+                md[0] = lane == 0 ? 0.0 : d;
+                mp[0] = lane == 0 ? 0.0 : x;
+            }
+        } else {
+            W[0] = o[0]; E[0] = o[1];
+            W[1] = o[1]; E[1] = __shfl_down_sync(0xffffffffu, o[0], 1);
+        }
+        double Bs[2] = {cone_sum(R, n.x, s.x, W[0], E[0]), cone_sum(R, n.y, s.y, W[1], E[1])};
+        double A[2] = {R.A, R.A}, r[2] = {R.rA, R.rA}, x[2];
+        if (special & (3u << (2 * P))) {
+            const uint32_t* f = B.info + c * B.ics + (la - 1) * WORDS + 2 * lane;
+            if (special & (1u << (2 * P))) Bs[0] = cone_special(B, R, f[0], Bs[0], n.x, s.x, W[0], E[0], A[0], r[0]);
+            if (special & (2u << (2 * P))) Bs[1] = cone_special(B, R, f[1], Bs[1], n.y, s.y, W[1], E[1], A[1], r[1]);
+        }
+        const bool act[2] = {(unsigned)tau - (unsigned)start[P][0] < t2, (unsigned)tau - (unsigned)start[P][1] < t2};
+        x[0] = quot(Bs[0], A[0], r[0]);
+        x[1] = quot(Bs[1], A[1], r[1]);
+        if ((act[0] && !(B.recip && sum_ok(Bs[0]))) || (act[1] && !(B.recip && sum_ok(Bs[1])))) {
+            x[0] = Bs[0] / A[0];
+            x[1] = Bs[1] / A[1];
+        }
+#pragma unroll
+        for (int w = 0; w < 2; w++) {
+            const double p = val[P][w], pn = p + CONE_OMEGA * (x[w] - p);
+            if (REDUCE) {
+                const double dch = fabs(pn - p), pabs = fabs(pn);
+                md[w] = act[w] && dch > md[w] ? dch : md[w];
+                mp[w] = act[w] && pabs > mp[w] ? pabs : mp[w];
+            }
+            val[P][w] = act[w] ? pn : p;
+        }
+        *reinterpret_cast<double2*>(B.phi + q[P]) = make_double2(val[P][0], val[P][1]);
+        if (edge) {
+            asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];"
+                         :: "r"(push + 8 * c * B.cs), "d"(val[P][0]), "d"(val[P][1]), "r"(bar_there + 8 * c) : "memory");
+            waiting = c;
+        }
+        if (REDUCE && P == 1 && tau >= e0 && (unsigned)(tau - e0) < t2) {
+            double2* slot = reinterpret_cast<double2*>(B.ring + 2 * ((((tau - e0) >> 1) + 1) & (B.R - 1)));
+            double2 cur = la == 1 ? make_double2(0.0, 0.0) : *slot;
+            const double d = (B.NK >> 1) & 1 ? md[1] : md[0], y = (B.NK >> 1) & 1 ? mp[1] : mp[0];
+            if (d > cur.x) cur.x = d;
+            if (y > cur.y) cur.y = y;
+            *slot = cur;
+        }
+    }
+    // the warp's row begins with phase 1: warps of such rows take their own copy of the solve
+    __device__ static bool odd_row(const Box& B) { return (B.A0 + 1 + (threadIdx.x >> 5)) & 1; }
+    template <bool PAR, int c, bool REDUCE>
+    __device__ __forceinline__ void step(const Box& B, int tau, unsigned t2) {
+        if (row_ok) phase<c ^ (int)PAR, c, REDUCE>(B, tau, t2);
+    }
+    __device__ __forceinline__ void end_step() { block_sync(); }
+};
 
 // s r D of a cell within H cells of the body: its 3-D face divergence with face values the
 // average of the two cells and zero through a face to a solid cell (InitValues_Jup.cpp:1653-1664).
@@ -259,52 +450,77 @@ __device__ double cone_face_div(const ConeArgs& A, int i, int j, int k) {
            (wp - wm) / A.dphi;
 }
 
-// the band's rows 1..nb of both colours between phi (colour stride cs) and a packed copy
-// [2][nb][PW] (to_packed) or back
+// the band and the rows beside it, 0..nb+1 of both colours, between phi (colour stride cs) and a packed
+// copy [2][nb + 2][PW] (to_packed) or back
 __device__ void band_copy(double* phi, int cs, double* packed, int nb, int PW, bool to_packed) {
-    const int n = 2 * nb * PW;
-    for (int x = threadIdx.x; x < n; x += blockDim.x) {
-        const int col = x / (nb * PW), r = x - col * nb * PW;
-        double* p = phi + col * cs + PW + r;      // local row 1 + r / PW, word r mod PW
-        if (to_packed) packed[x] = *p;
-        else *p = packed[x];
-    }
+    const int n = (nb + 2) * PW;
+    for (int col = 0; col < 2; col++)
+        for (int x = threadIdx.x; x < n; x += blockDim.x) {
+            if (to_packed) packed[col * n + x] = phi[col * cs + x];
+            else phi[col * cs + x] = packed[col * n + x];
+        }
 }
 
 // Lexicographic SOR of one level's solve as the pipelined wavefront on the cluster; returns the
 // reference's sweep count `it` (the converged sweep, or CONE_MAXIT + 1 without convergence).
-// snap: this block's snapshot ring, n_snap slots of 2 nbmax PW doubles. A cluster barrier ends
-// every step: the next step's edge rows read the neighbours' rows of this one.
-__device__ int cone_sor(const Box& B, double* snap, int slot_sz, int n_snap, int* snap_tag, int C) {
+// snap: this block's snapshot ring, n_snap slots of 2 (nbmax + 2) PW doubles.
+template <class Form, bool PAR>
+__device__ __forceinline__ int cone_sor(const Box& B, Form& T, double* snap, int slot_sz, int n_snap, int* snap_tag, int* t_found, int C) {
     cg::cluster_group cl = cg::this_cluster();
+    const int lane = threadIdx.x & 31;
+    cluster_sync();              // the cluster's blocks hold their start: a neighbour may store its edge row here
     band_copy(B.phi, B.cs, snap, B.nb, B.PW, true);
     if (threadIdx.x == 0) {
         snap_tag[0] = -1;
         for (int s = 1; s < n_snap; s++) snap_tag[s] = INT_MIN;
     }
-    cl.sync();
-    int next = 1 % n_snap, t_conv = 0, it = CONE_MAXIT + 1;
-    for (int tau = 0;; tau++) {
-        cone_step(B, tau, CONE_MAXIT, true);
-        cl.sync();
-        if (tau >= B.D && ((tau - B.D) & 1) == 0) {
-            const int t = (tau - B.D) / 2 + 1;       // the sweep this step completed
-            double dmax = 0.0, pmax = 0.0;
-            for (int r = 0; r < C; r++) {
-                const unsigned long long* sl = cl.map_shared_rank(B.ring + 2 * (t & (B.R - 1)), r);
-                dmax = fmax(dmax, __longlong_as_double((long long)sl[0]));
-                pmax = fmax(pmax, __longlong_as_double((long long)sl[1]));
+    cluster_sync();
+    T.init(B);
+    int next = 1 % n_snap, t_conv = 0, t_next = 1, it = CONE_MAXIT + 1;
+    for (int tau = 1;; tau += 2) {
+        T.template step<PAR, 0, true>(B, tau - 1, 2u * CONE_MAXIT);
+        T.end_step();
+        T.template step<PAR, 1, true>(B, tau, 2u * CONE_MAXIT);
+        T.end_step();
+        // a sweep's last raise comes up to one step after its last cell
+        if (tau > B.D && (tau & (CHECK_STEPS - 1)) == CHECK_STEPS - 1) {
+            // the sweeps t_next..t_done are complete, at most CHECK_STEPS / 2 of them: lane 4 q + r of
+            // the first warp reads block r's slot of sweep t_next + q
+            const int t_done = min((tau - B.D - 1) / 2 + 1, CONE_MAXIT);
+            cluster_sync();      // the blocks' ring slots are theirs to read
+            if (threadIdx.x < 32) {
+                const int t = t_next + (lane >> 2);
+                double dmax = 0.0, pmax = 0.0;
+                if (t <= t_done && (lane & 3) < C) {
+                    const double2 sl = *reinterpret_cast<const double2*>(
+                        cl.map_shared_rank(B.ring + 2 * (t & (B.R - 1)), lane & 3));
+                    dmax = sl.x;
+                    pmax = sl.y;
+                }
+                for (int o = 1; o < 4; o <<= 1) {
+                    dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+                    pmax = fmax(pmax, __shfl_xor_sync(0xffffffffu, pmax, o));
+                }
+                const unsigned conv = __ballot_sync(0xffffffffu, t <= t_done && dmax <= CONE_TOL * fmax(pmax, 1.0e-30));
+                if (lane == 0) *t_found = conv ? t_next + ((__ffs(conv) - 1) >> 2) : 0;
             }
-            if (dmax <= CONE_TOL * fmax(pmax, 1.0e-30)) { t_conv = t; break; }
-            if (t == CONE_MAXIT) break;
+            block_sync();
+            t_conv = *t_found;
+            if (t_conv > 0) break;
+            t_next = t_done + 1;
+            if (t_done == CONE_MAXIT) break;
         }
         if (tau % SNAP_EVERY == SNAP_EVERY - 1) {
+            T.settle(B);
+            block_sync();
             band_copy(B.phi, B.cs, snap + (size_t)next * slot_sz, B.nb, B.PW, true);
             if (threadIdx.x == 0) snap_tag[next] = tau;
             next = (next + 1) % n_snap;
-            __syncthreads();
+            cluster_sync();      // the copies of the neighbours' rows are saved before the next step's stores
         }
     }
+    T.settle(B);
+    block_sync();
     if (t_conv > 0) {
         // back to the newest snapshot in which no cell is past sweep t_conv (the same slot in
         // every block), then replay with the sweeps capped at t_conv up to the step that
@@ -315,18 +531,25 @@ __device__ int cone_sor(const Box& B, double* snap, int slot_sz, int n_snap, int
         for (int s = 0; s < n_snap; s++)
             if (snap_tag[s] != INT_MIN && snap_tag[s] <= target && snap_tag[s] > btag) { best = s; btag = snap_tag[s]; }
         band_copy(B.phi, B.cs, snap + (size_t)best * slot_sz, B.nb, B.PW, false);
-        cl.sync();
-        for (int tau = btag + 1; tau <= tau_c; tau++) {
-            cone_step(B, tau, t_conv, false);
-            cl.sync();
+        cluster_sync();
+        T.load(B);
+        for (int tau = btag + 1; tau <= tau_c; tau += 2) {     // from an even step; one past tau_c changes nothing
+            T.template step<PAR, 0, false>(B, tau, 2u * t_conv);
+            T.end_step();
+            T.template step<PAR, 1, false>(B, tau + 1, 2u * t_conv);
+            T.end_step();
         }
+        T.settle(B);
+        block_sync();
     }
     return it;
 }
 
-__global__ void __launch_bounds__(CONE_THREADS, 1) cone_kernel(ConeArgs A) {
+// SMEM: phi, flags and constants of the band in shared memory; else one block per level on HBM
+template <bool SMEM, class Form>
+__global__ void __launch_bounds__(Form::THREADS, 1) cone_kernel(ConeArgs A) {
     extern __shared__ __align__(16) unsigned char cone_smem[];
-    __shared__ int snap_tag[64];
+    __shared__ int snap_tag[64], t_found;
     cg::cluster_group cl = cg::this_cluster();
     const int C = A.C;
     const int r = (int)cl.block_rank();
@@ -338,28 +561,37 @@ __global__ void __launch_bounds__(CONE_THREADS, 1) cone_kernel(ConeArgs A) {
     B.NJ = NJ; B.NK = NK; B.PW = PW; B.D = L.D; B.R = L.ring;
     B.nb = nb; B.A0 = A0;
     B.dthe = A.dthe; B.dphi = A.dphi;
-    B.lgCH = 0;
-    while ((32 << B.lgCH) < PW) B.lgCH++;
     B.ring = reinterpret_cast<unsigned long long*>(cone_smem);
     double* phi_local = reinterpret_cast<double*>(B.ring + 2 * A.ring_max);
     double *rows, *tab;
-    if (A.smem_mode) {
+    B.push_n = B.push_s = nullptr;
+    __shared__ __align__(8) unsigned long long bars[4];        // north's two colours, south's two
+    Form T;
+    if constexpr (std::is_same<Form, RowForm>::value) {
+        B.bar = (unsigned)__cvta_generic_to_shared(bars);
+        T.phases = 0;
+        T.dead = false;
+        if (threadIdx.x == 0) {
+            for (int x = 0; x < 4; x++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(B.bar + 8 * x) : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        // a row stored in the neighbour to the north is that block's southern one
+        if (r > 0) B.bar_n = (unsigned)__cvta_generic_to_shared(cl.map_shared_rank(bars + 2, r - 1));
+        if (r < C - 1) B.bar_s = (unsigned)__cvta_generic_to_shared(cl.map_shared_rank(bars, r + 1));
+    }
+    if constexpr (SMEM) {
         B.cs = (nbmax + 2) * PW;
         rows = phi_local + 2 * B.cs;
         tab = rows + NROW * NJ;
-        uint32_t* inf = reinterpret_cast<uint32_t*>(tab + 2 * L.n_spec);
+        uint32_t* inf = reinterpret_cast<uint32_t*>(tab + L.n_tab);
         B.ics = nbmax * PW;
         for (int x = threadIdx.x; x < 2 * nb * PW; x += blockDim.x) {
             const int col = x / (nb * PW), rr = x - col * nb * PW;
             inf[col * B.ics + rr] = A.info[L.info_off + (size_t)col * NJ * PW + (size_t)A0 * PW + rr];
         }
         B.info = inf;
-        for (int x = 0; x < 2; x++) {
-            B.nrow[x] = r > 0 ? cl.map_shared_rank(phi_local + x * B.cs + (A0 - ((r - 1) * NJ) / C) * PW, r - 1)
-                              : phi_local + x * B.cs;
-            B.srow[x] = r < C - 1 ? cl.map_shared_rank(phi_local + x * B.cs + PW, r + 1)
-                                  : phi_local + x * B.cs + (nb + 1) * PW;
-        }
+        if (r > 0) B.push_n = cl.map_shared_rank(phi_local + (A0 - ((r - 1) * NJ) / C + 1) * PW, r - 1);
+        if (r < C - 1) B.push_s = cl.map_shared_rank(phi_local, r + 1);
     } else {
         // one block per level: phi in place in the warm-start buffer, the rest in HBM
         B.cs = (NJ + 2) * PW;
@@ -371,6 +603,7 @@ __global__ void __launch_bounds__(CONE_THREADS, 1) cone_kernel(ConeArgs A) {
     B.tab = tab;
     B.rows = rows;
     // the row coefficients (InitValues_Jup.cpp:1733-1735) and A of a cell with four fluid faces
+    bool recip = true;
     for (int a = threadIdx.x; a < NJ; a += blockDim.x) {
         const int j = L.jlo + a;
         const double sj = A.s[j];
@@ -382,37 +615,32 @@ __global__ void __launch_bounds__(CONE_THREADS, 1) cone_kernel(ConeArgs A) {
         a4 += aS;
         a4 += aL;
         a4 += aL;
-        rows[a] = aN;
-        rows[NJ + a] = aS;
-        rows[2 * NJ + a] = aL;
-        rows[3 * NJ + a] = sj;
-        rows[4 * NJ + a] = sj * A.dphi;
-        rows[5 * NJ + a] = a4;
+        double* rc = rows + (size_t)a * NROW;
+        rc[RC_N] = aN;
+        rc[RC_S] = aS;
+        rc[RC_L] = aL;
+        rc[RC_A] = a4;
+        rc[RC_RA] = rcp_of(a4);
+        rc[RC_SJ] = sj;
+        rc[RC_SD] = sj * A.dphi;
+        recip = recip && aN > 0.0 && aS > 0.0 && aL > 0.0 && quot_ok(1.0, aN) && quot_ok(1.0, aS) && quot_ok(1.0, aL) && quot_ok(1.0, a4);
     }
+    B.recip = __syncthreads_and(recip) != 0;
     const int32_t* spec = A.spec + L.spec_off;
-    const int slot_sz = 2 * nbmax * PW;
+    const int slot_sz = 2 * (nbmax + 2) * PW;
     double* snap = A.snap + L.snap_off + (size_t)r * L.n_snap * slot_sz;
     if (A.H == 0 && r == 0 && threadIdx.x == 0) A.stats[2 * lvl] = 0;
     for (int pass = A.H > 0 ? 0 : 1; pass < 2; pass++) {
         B.div = pass == 0;
         double* prev = (B.div ? A.prev0 : A.prev1) + L.phi_off;
-        if (A.smem_mode) {
+        if constexpr (SMEM) {
+            // the band with the rows beside it (zero at the box's halo)
             B.phi = phi_local;
-            for (int x = threadIdx.x; x < 2 * PW; x += blockDim.x) {   // the rows beside the band
-                const int col = x / PW, mm = x - col * PW;
-                phi_local[col * B.cs + mm] = 0.0;
-                phi_local[col * B.cs + (nb + 1) * PW + mm] = 0.0;
-            }
-            for (int x = threadIdx.x; x < 2 * nb * PW; x += blockDim.x) {
-                const int col = x / (nb * PW), rr = x - col * nb * PW;
-                phi_local[col * B.cs + PW + rr] = prev[(size_t)col * (NJ + 2) * PW + (size_t)(A0 + 1) * PW + rr];
-            }
+            for (int col = 0; col < 2; col++)
+                for (int x = threadIdx.x; x < (nb + 2) * PW; x += blockDim.x)
+                    phi_local[col * B.cs + x] = prev[(size_t)col * (NJ + 2) * PW + (size_t)A0 * PW + x];
         } else {
             B.phi = prev + (size_t)A0 * PW;
-            for (int x = 0; x < 2; x++) {
-                B.nrow[x] = B.phi + x * B.cs;
-                B.srow[x] = B.phi + x * B.cs + (nb + 1) * PW;
-            }
         }
         // the per-cell constants of the band: the source of the divergence solve from the flow
         // before it, the wall-face velocities of the wall-flux solve from the flow it starts from
@@ -422,15 +650,29 @@ __global__ void __launch_bounds__(CONE_THREADS, 1) cone_kernel(ConeArgs A) {
             if (a < A0 || a >= A0 + nb) continue;
             const int b = ((cc ^ (a + 1)) & 1) + 2 * mm - 1;
             const int j = L.jlo + a, k = L.klo + b;
-            if (B.div) {
-                tab[2 * x] = (A.info[L.info_off + e] & CF_NEAR) ? cone_face_div(A, i, j, k) : 0.0;
-            } else {
-                const size_t cix = ((size_t)i * A.jm + j) * A.KP + k;
-                tab[2 * x] = A.v[cix];
-                tab[2 * x + 1] = A.w[cix];
-            }
+            const uint32_t f = A.info[L.info_off + e];
+            double* t = tab + 2 * (f >> 6);
+            const double src = B.div && (f & CF_NEAR) ? cone_face_div(A, i, j, k) : 0.0;
+            if (!(f & CF_WALL)) { t[0] = src; continue; }
+            const double* rc = rows + (size_t)a * NROW;
+            double sum = 0.0;
+            if (!(f & CF_N)) sum += rc[RC_N];
+            if (!(f & CF_S)) sum += rc[RC_S];
+            if (!(f & CF_W)) sum += rc[RC_L];
+            if (!(f & CF_E)) sum += rc[RC_L];
+            t[0] = sum;
+            t[1] = rcp_of(sum);
+            const size_t cix = ((size_t)i * A.jm + j) * A.KP + k;
+            const double vp = A.v[cix], wp = A.w[cix], sj = rc[RC_SJ];
+            t[2] = B.div ? 0.0 : -(rc[RC_N] * A.dthe * (-vp));
+            t[3] = B.div ? 0.0 : -(rc[RC_S] * A.dthe * (vp));
+            t[4] = B.div ? 0.0 : -(rc[RC_L] * sj * A.dphi * (-wp));
+            t[5] = B.div ? 0.0 : -(rc[RC_L] * sj * A.dphi * (wp));
+            t[6] = src;
         }
-        const int it = cone_sor(B, snap, slot_sz, L.n_snap, snap_tag, C);
+        const int it = Form::odd_row(B) ? cone_sor<Form, true>(B, T, snap, slot_sz, L.n_snap, snap_tag, &t_found, C)
+                                        : cone_sor<Form, false>(B, T, snap, slot_sz, L.n_snap, snap_tag, &t_found, C);
+        __syncthreads();
         // v and w of the band incremented by the average of the two face corrections
         // (InitValues_Jup.cpp:1785-1793), a wall face's correction being minus the cell's velocity
         for (int x = threadIdx.x; x < nb * NK; x += blockDim.x) {
@@ -440,7 +682,7 @@ __global__ void __launch_bounds__(CONE_THREADS, 1) cone_kernel(ConeArgs A) {
             if (inf & CF_SOLID) continue;
             const size_t cix = ((size_t)i * A.jm + (L.jlo + a)) * A.KP + (L.klo + b);
             const double vp = A.v[cix], wp = A.w[cix], pp = phi_at(B, la, bp);
-            const double sd = rows[4 * NJ + a];
+            const double sd = rows[(size_t)a * NROW + RC_SD];
             const double dN = (inf & CF_N) ? -vp : (pp - phi_at(B, la - 1, bp)) / A.dthe;
             const double dS = (inf & CF_S) ? -vp : (phi_at(B, la + 1, bp) - pp) / A.dthe;
             const double dW = (inf & CF_W) ? -wp : (pp - phi_at(B, la, bp - 1)) / sd;
@@ -449,14 +691,16 @@ __global__ void __launch_bounds__(CONE_THREADS, 1) cone_kernel(ConeArgs A) {
             A.w[cix] = wp + 0.5 * (dW + dE);
         }
         // the band's phi is the warm start of the next call
-        if (A.smem_mode)
+        if constexpr (SMEM)
             for (int x = threadIdx.x; x < 2 * nb * PW; x += blockDim.x) {
                 const int col = x / (nb * PW), rr = x - col * nb * PW;
                 prev[(size_t)col * (NJ + 2) * PW + (size_t)(A0 + 1) * PW + rr] = phi_local[col * B.cs + PW + rr];
             }
         if (r == 0 && threadIdx.x == 0) A.stats[2 * lvl + pass] = it;
-        // the neighbours have read this band's edge rows before the next pass overwrites them
+        const bool lost = __syncthreads_or(!T.settle(B)) != 0;      // a neighbour's row never came
+        // every block is past its last store to a neighbour, and the warm start is read after it is whole
         cl.sync();
+        if (lost && threadIdx.x == 0) A.stats[2 * lvl + pass] = -1;
     }
 }
 
@@ -561,10 +805,12 @@ int cone_prepare(AtjupCtx* c) {
         ConeLevel L{};
         L.i = i; L.jlo = jlo; L.klo = klo;
         L.NJ = jhi - jlo + 1; L.NK = khi - klo + 1;
-        L.PW = (L.NK + 3) / 2;                       // words per row and colour, halo included
+        // words per row and colour, halo included; RowForm's lanes have all their words in every row
+        L.PW = std::max((L.NK + 3) / 2, RowForm::WORDS);
         L.D = L.NJ + L.NK - 2;
         L.ring = 1;
-        while (L.ring < L.D / 2 + 2) L.ring <<= 1;     // a power of two above the sweeps in flight
+        // a power of two above the sweeps in flight and those that wait for their stopping test
+        while (L.ring < L.D / 2 + 4 + CHECK_STEPS / 2) L.ring <<= 1;
         L.n_snap = (L.D + SNAP_EVERY) / SNAP_EVERY + 2;
         if (L.n_snap > 64 || L.PW > 32 * 32) {
             delete cs;
@@ -587,7 +833,9 @@ int cone_prepare(AtjupCtx* c) {
                     if (S(i, j, k + 1)) f |= CF_E;
                     if (H > 0 && near[((size_t)i * jm + j) * km + k]) f |= CF_NEAR;
                     if (f) {
-                        f |= (uint32_t)(spec.size() - L.spec_off) << 6;
+                        const int entry = f & CF_WALL ? TAB_WALL : TAB_NEAR;
+                        f |= (uint32_t)(L.n_tab / 2) << 6;
+                        L.n_tab += entry;
                         spec.push_back(e);
                     }
                 }
@@ -596,7 +844,7 @@ int cone_prepare(AtjupCtx* c) {
         L.n_spec = (int)(spec.size() - L.spec_off);
         const int64_t nphi = 2 * (int64_t)(L.NJ + 2) * L.PW;
         L.phi_off = n_phi;  n_phi += nphi;
-        L.tab_off = n_tab;  n_tab += 2 * (int64_t)L.n_spec;
+        L.tab_off = n_tab;  n_tab += L.n_tab;
         L.row_off = n_row;  n_row += NROW * (int64_t)L.NJ;
         cs->ring_max = std::max(cs->ring_max, L.ring);
         cs->lv.push_back(L);
@@ -613,10 +861,24 @@ int cone_prepare(AtjupCtx* c) {
         for (const ConeLevel& L : cs->lv) {
             const size_t nbmax = (size_t)(L.NJ + Cn - 1) / Cn;
             mx = std::max(mx, sizeof(double) * (2 * (nbmax + 2) * L.PW + NROW * (size_t)L.NJ +
-                                                2 * (size_t)L.n_spec) +
+                                                (size_t)L.n_tab) +
                                   sizeof(uint32_t) * 2 * nbmax * L.PW);
         }
         return mx + sizeof(unsigned long long) * 2 * (size_t)cs->ring_max;
+    };
+    // the kernel for C blocks a level and its threads: a warp per row where every band allows it
+    auto form_for = [&](int Cn, int& threads) {
+        int rows = 1, words = 1, least = INT_MAX;
+        for (const ConeLevel& L : cs->lv) {
+            rows = std::max(rows, (L.NJ + Cn - 1) / Cn);
+            words = std::max(words, L.PW);
+            least = std::min(least, L.NJ / Cn);
+        }
+        const bool row = cs->smem_mode && least >= 2 && rows <= RowForm::ROWS && words <= RowForm::WORDS;
+        threads = row ? 32 * rows : WordForm::THREADS;
+        return row ? reinterpret_cast<const void*>(&cone_kernel<true, RowForm>)
+                   : cs->smem_mode ? reinterpret_cast<const void*>(&cone_kernel<true, WordForm>)
+                                   : reinterpret_cast<const void*>(&cone_kernel<false, WordForm>);
     };
     cs->smem_mode = nl > 0 && smem_for(std::max(C, 1)) <= CONE_SMEM_CAP;
     if (!cs->smem_mode) C = 1;
@@ -625,7 +887,9 @@ int cone_prepare(AtjupCtx* c) {
     for (; nl > 0 && C > 1; C--) {
         const size_t sm = smem_for(C);
         if (sm > CONE_SMEM_CAP) continue;
-        if (cudaFuncSetAttribute(cone_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) {
+        int threads = 0;
+        const void* form = form_for(C, threads);
+        if (cudaFuncSetAttribute(form, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) {
             cudaGetLastError();
             continue;
         }
@@ -634,24 +898,25 @@ int cone_prepare(AtjupCtx* c) {
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.gridDim = dim3((unsigned)(nl * C));
-        cfg.blockDim = dim3(CONE_THREADS);
+        cfg.blockDim = dim3(threads);
         cfg.dynamicSmemBytes = sm;
         cfg.attrs = at;
         cfg.numAttrs = 1;
         int n_active = 0;
-        if (cudaOccupancyMaxActiveClusters(&n_active, cone_kernel, &cfg) == cudaSuccess &&
+        if (cudaOccupancyMaxActiveClusters(&n_active, form, &cfg) == cudaSuccess &&
             n_active >= (int)nl)
             break;
         cudaGetLastError();
     }
     cs->smem = cs->smem_mode ? smem_for(C) : sizeof(unsigned long long) * 2 * (size_t)cs->ring_max;
+    cs->kernel = form_for(C, cs->threads);
     if (nl > 0)
-        ATJUP_CUDA(cudaFuncSetAttribute(cone_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cs->smem));
+        ATJUP_CUDA(cudaFuncSetAttribute(cs->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cs->smem));
     cs->C = C;
     for (ConeLevel& L : cs->lv) {
         const int64_t nbmax = (L.NJ + C - 1) / C;
         L.snap_off = n_snap;
-        n_snap += (int64_t)C * L.n_snap * 2 * nbmax * L.PW;
+        n_snap += (int64_t)C * L.n_snap * 2 * (nbmax + 2) * L.PW;
     }
     ATJUP_CUDA(cudaMalloc(&cs->s, sizeof(double) * jm));
     ATJUP_CUDA(cudaMemcpy(cs->s, s.data(), sizeof(double) * jm, cudaMemcpyHostToDevice));
@@ -690,7 +955,6 @@ int launch_cone_projection(AtjupCtx* c) {
         A.u = c->f[ATJUP_F_U]; A.v = c->f[ATJUP_F_V]; A.w = c->f[ATJUP_F_W];
         A.solid = c->solid; A.rad = c->rad;
         A.jm = P.jm; A.km = P.km; A.KP = c->KP; A.H = cs->H;
-        A.smem_mode = cs->smem_mode;
         A.C = cs->C;
         A.ring_max = cs->ring_max;
         A.dr = P.dr; A.dthe = P.dthe; A.dphi = P.dphi;
@@ -699,13 +963,14 @@ int launch_cone_projection(AtjupCtx* c) {
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = cs->C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.gridDim = dim3((unsigned)(cs->lv.size() * cs->C));
-        cfg.blockDim = dim3(CONE_THREADS);
+        cfg.blockDim = dim3(cs->threads);
         cfg.dynamicSmemBytes = cs->smem;
         cfg.stream = c->stream;
         cfg.attrs = at;
         cfg.numAttrs = 1;
         c->launches++;
-        ATJUP_CUDA(cudaLaunchKernelEx(&cfg, cone_kernel, A));
+        void* args[] = {&A};
+        ATJUP_CUDA(cudaLaunchKernelExC(&cfg, cs->kernel, args));
         ATJUP_CHECK_LAUNCH("cone projection");
     }
     const int rows = P.im * P.jm;

@@ -14,6 +14,7 @@
 // finishes; cells of one warp share i and j and differ only in longitude, so they tend to take
 // the same branch.
 #include "ctx.cuh"
+#include "quot.cuh"
 
 namespace atjup {
 namespace {
@@ -21,17 +22,43 @@ namespace {
 constexpr int SAT_PASSES = 15;          // iter_prec_end (SaturationAdjustment.h:250)
 constexpr double SAT_Q_DIFF_MIN = 1.0e-3;  // q_diff_min (SaturationAdjustment.h:251)
 
-// ATPhys::saturation_vapour_pressure (ATPhys.h:49-52) [bar]
-__device__ __forceinline__ double svp(double T, double C, double L0, double R, double da,
-                                      double db) {
-    return exp(C + (-L0 / T + da * log(T) + db * T) / (1e-3 * R));
-}
+// A cell's saturation densities ((rho ep) E(T)) / p_u, the reference's rho_c * ep * E / p_u, E the saturation
+// vapour pressure [bar] (ATPhys.h:49-52). The quotients are by T, by the constant 1e-3 R and by p_u, each by
+// one reciprocal for both phases (quot.cuh), and both share the logarithm: one after another the
+// divisions were most of a pass.
+struct Curve {
+    double rep, p_u, p_r, kR, kR_r;
+    __device__ __forceinline__ double one(double T, double C, double L0, double da, double db) const {
+        const double x = quot1_by(quot1(-L0, T) + da * log(T) + db * T, kR, kR_r);
+        return quot1_by(rep * exp(C + x), p_u, p_r);
+    }
+    __device__ __forceinline__ double liquid(const AtjupGasParams& g, double T) const {
+        return one(T, g.C, g.L0, g.del_alf, g.del_bet);
+    }
+    __device__ __forceinline__ double ice(const AtjupGasParams& g, double T) const {
+        return one(T, g.C_i, g.L0_i, g.del_alf_i, g.del_bet_i);
+    }
+    __device__ __forceinline__ void both(const AtjupGasParams& g, double T, double& ql, double& qs) const {
+        const double lT = log(T);
+        const double L[2] = {-g.L0, -g.L0_i};
+        double x[2], n[2], q[2];
+        quots_by(L, T, rcp_of(T), x);
+        n[0] = x[0] + g.del_alf * lT + g.del_bet * T;
+        n[1] = x[1] + g.del_alf_i * lT + g.del_bet_i * T;
+        quots_by(n, kR, kR_r, x);
+        n[0] = rep * exp(g.C + x[0]);
+        n[1] = rep * exp(g.C_i + x[1]);
+        quots_by(n, p_u, p_r, q);
+        ql = q[0];
+        qs = q[1];
+    }
+};
 
 // Vapour target for q_c liquid and q_i ice at T from the liquid / ice saturation densities
 // (SaturationAdjustment.h:513-520; the Newton probe at 564-571 makes the same choice).
 __device__ __forceinline__ double target(const AtjupGasParams& g, double T, double qc, double qi,
                                          double ql, double qs, double tri) {
-    if (qc > 0.0 && qi > 0.0) return (qc * ql + qi * qs) / (qc + qi);
+    if (qc > 0.0 && qi > 0.0) return quot1(qc * ql + qi * qs, qc + qi);
     if (g.bergeron >= 2 && qc <= 0.0 && qi <= 0.0 && T < g.t_0) return qs;
     if (g.ice_entry && qc <= 0.0 && qi <= 0.0) {
         const double cn = T <= g.t_00 ? 0.0 : (T >= g.t_0 ? 1.0 : (T - g.t_00) * tri);
@@ -51,6 +78,7 @@ struct SatArgs {
     long long ncell_padded;
     int KP, km, local_rho;
     double t_ref, r_mix, cp_mix;
+    double tri, kR, kR_r, t_ref_r;    // 1 / (t_0 - t_00), 1e-3 R and its reciprocal, 1 / t_ref
 };
 
 __global__ void __launch_bounds__(256) satadj_kernel(SatArgs a, AtjupGasParams g) {
@@ -63,7 +91,7 @@ __global__ void __launch_bounds__(256) satadj_kernel(SatArgs a, AtjupGasParams g
         const double c_in = c, cl_in = cl, ic_in = ic;
         bool t_dirty = false;
         double t_out = 0.0;
-        const double tri = 1.0 / (g.t_0 - g.t_00);
+        const double tri = a.tri;
         const double Lf = g.ls - g.lv;
         bool active = (t_u > 0.0) && (p_u > 0.0) && !a.solid[q];
         if (active) {
@@ -72,17 +100,17 @@ __global__ void __launch_bounds__(256) satadj_kernel(SatArgs a, AtjupGasParams g
                 const double r = a.rho_mix[q];
                 if (r > 0.0 && isfinite(r)) rho = r;
             }
-            const double heat = a.cp_mix * rho;
+            const double heat = a.cp_mix * rho, heat_r = rcp_of(heat);
             // entry bounds: melt above t_0, optional freeze below t_00, clip negatives
             if (t_u > g.t_0) {
                 if (g.conserve) {
                     if (ic > 0.0) {
                         double dm = ic;
                         if (Lf > 0.0) {
-                            const double cap = heat * (t_u - g.t_0) / Lf;
+                            const double cap = quot1(heat * (t_u - g.t_0), Lf);
                             if (dm > cap) dm = cap;
-                            t_u -= Lf * dm / heat;
-                            t_out = t_u / a.t_ref;
+                            t_u -= quot1_by(Lf * dm, heat, heat_r);
+                            t_out = quot1_by(t_u, a.t_ref, a.t_ref_r);
                             t_dirty = true;
                         }
                         ic -= dm;
@@ -96,10 +124,10 @@ __global__ void __launch_bounds__(256) satadj_kernel(SatArgs a, AtjupGasParams g
                 cl > 0.0) {
                 double dm = cl;
                 if (Lf > 0.0) {
-                    const double cap = heat * (g.t_00 - t_u) / Lf;
+                    const double cap = quot1(heat * (g.t_00 - t_u), Lf);
                     if (dm > cap) dm = cap;
-                    t_u += Lf * dm / heat;
-                    t_out = t_u / a.t_ref;
+                    t_u += quot1_by(Lf * dm, heat, heat_r);
+                    t_out = quot1_by(t_u, a.t_ref, a.t_ref_r);
                     t_dirty = true;
                 }
                 cl -= dm;
@@ -109,10 +137,9 @@ __global__ void __launch_bounds__(256) satadj_kernel(SatArgs a, AtjupGasParams g
             if (cl < 0.0) cl = 0.0;
             if (ic < 0.0) ic = 0.0;
 
-            // entry test (SaturationAdjustment.h:422-452); every saturation density is
-            // ((rho * ep) * E) / p_u, the reference's rho_c * ep * E / p_u
-            const double rep = rho * g.ep;
-            const double q_rain0 = rep * svp(t_u, g.C, g.L0, g.R, g.del_alf, g.del_bet) / p_u;
+            // entry test (SaturationAdjustment.h:422-452)
+            const Curve sat{rho * g.ep, p_u, rcp_of(p_u), a.kR, a.kR_r};
+            const double q_rain0 = sat.liquid(g, t_u);
             bool enter = q_rain0 > 0.0;
             if (enter) {
                 double q_entry = q_rain0;
@@ -120,19 +147,17 @@ __global__ void __launch_bounds__(256) satadj_kernel(SatArgs a, AtjupGasParams g
                     const double cnd0 = t_u <= g.t_00 ? 0.0
                                       : (t_u >= g.t_0 ? 1.0 : (t_u - g.t_00) * tri);
                     if (cnd0 < 1.0)
-                        q_entry = cnd0 * q_rain0 + (1.0 - cnd0) * rho * g.ep
-                                * svp(t_u, g.C_i, g.L0_i, g.R, g.del_alf_i, g.del_bet_i) / p_u;
+                        q_entry = cnd0 * q_rain0 + Curve{(1.0 - cnd0) * rho * g.ep, p_u, sat.p_r, a.kR, a.kR_r}.ice(g, t_u);
                 }
                 if (g.bergeron >= 2 && cl <= 0.0 && ic <= 0.0 && t_u < g.t_0)
-                    q_entry = rep * svp(t_u, g.C_i, g.L0_i, g.R, g.del_alf_i, g.del_bet_i) / p_u;
+                    q_entry = sat.ice(g, t_u);
                 if (c <= q_entry) {
                     if (!g.evap || !g.conserve || (cl <= 0.0 && ic <= 0.0)) {
                         enter = false;
                     } else {
-                        const double q_ice0 =
-                            rep * svp(t_u, g.C_i, g.L0_i, g.R, g.del_alf_i, g.del_bet_i) / p_u;
+                        const double q_ice0 = sat.ice(g, t_u);
                         double q_t0;
-                        if (cl > 0.0 && ic > 0.0) q_t0 = (cl * q_rain0 + ic * q_ice0) / (cl + ic);
+                        if (cl > 0.0 && ic > 0.0) q_t0 = quot1(cl * q_rain0 + ic * q_ice0, cl + ic);
                         else if (ic <= 0.0) q_t0 = q_rain0;
                         else q_t0 = q_ice0;
                         if (fabs(c - q_t0) <= SAT_Q_DIFF_MIN * q_t0) enter = false;
@@ -155,7 +180,7 @@ __global__ void __launch_bounds__(256) satadj_kernel(SatArgs a, AtjupGasParams g
                         CND = 0.0;
                         DEP = 1.0;
                         if (qc > 0.0) {
-                            T -= g.lv * qc / heat;
+                            T -= quot1_by(g.lv * qc, heat, heat_r);
                             qv += qc;
                             qc = 0.0;
                         }
@@ -174,7 +199,7 @@ __global__ void __launch_bounds__(256) satadj_kernel(SatArgs a, AtjupGasParams g
                         }
                         dv = -(dc + di);
                     }
-                    T += (g.lv * dc + g.ls * di) / heat;
+                    T += quot1_by(g.lv * dc + g.ls * di, heat, heat_r);
                     qv += dv;
                     qc += dc;
                     qi += di;
@@ -182,9 +207,8 @@ __global__ void __launch_bounds__(256) satadj_kernel(SatArgs a, AtjupGasParams g
                     if (qc < 0.0) qc = 0.0;
                     if (qi < 0.0) qi = 0.0;
 
-                    const double ql = rep * svp(T, g.C, g.L0, g.R, g.del_alf, g.del_bet) / p_u;
-                    const double qs =
-                        rep * svp(T, g.C_i, g.L0_i, g.R, g.del_alf_i, g.del_bet_i) / p_u;
+                    double ql, qs;
+                    sat.both(g, T, ql, qs);
                     q_rain_now = ql;
                     hyp = target(g, T, qc, qi, ql, qs, tri);
 
@@ -193,9 +217,9 @@ __global__ void __launch_bounds__(256) satadj_kernel(SatArgs a, AtjupGasParams g
                             if (qi > 0.0) {
                                 double dm = qi;
                                 if (Lf > 0.0) {
-                                    const double cap = heat * (T - g.t_0) / Lf;
+                                    const double cap = quot1(heat * (T - g.t_0), Lf);
                                     if (dm > cap) dm = cap;
-                                    T -= Lf * dm / heat;
+                                    T -= quot1_by(Lf * dm, heat, heat_r);
                                 }
                                 qi -= dm;
                                 qc += dm;
@@ -204,7 +228,7 @@ __global__ void __launch_bounds__(256) satadj_kernel(SatArgs a, AtjupGasParams g
                             qi = 0.0;
                         }
                     }
-                    const double q_diff = fabs(qv - hyp) / (hyp + 1e-20);
+                    const double q_diff = quot1(fabs(qv - hyp), hyp + 1e-20);
                     if (q_diff <= SAT_Q_DIFF_MIN) { found = true; break; }
                     if (g.dry_exit && g.conserve && qc <= 0.0 && qi <= 0.0 && qv < hyp) {
                         dry = true;
@@ -212,18 +236,16 @@ __global__ void __launch_bounds__(256) satadj_kernel(SatArgs a, AtjupGasParams g
                     }
                     if (g.newton) {
                         const double dT = 0.1;
-                        const double qld =
-                            rep * svp(T + dT, g.C, g.L0, g.R, g.del_alf, g.del_bet) / p_u;
-                        const double qsd =
-                            rep * svp(T + dT, g.C_i, g.L0_i, g.R, g.del_alf_i, g.del_bet_i) / p_u;
+                        double qld, qsd;
+                        sat.both(g, T + dT, qld, qsd);
                         const double hyp_d = target(g, T, qc, qi, qld, qsd, tri);
                         double CNDn = (T - g.t_00) * tri;
                         if (T <= g.t_00) CNDn = 0.0;
                         if (T >= g.t_0) CNDn = 1.0;
                         if (berg) CNDn = 0.0;
-                        const double G = (g.lv * CNDn + g.ls * (1.0 - CNDn)) / heat *
-                                         (hyp_d - hyp) / dT;
-                        double w = 1.0 / (1.0 + (G < 0.0 ? 0.0 : G));
+                        const double G = quot1_by(quot1_by(g.lv * CNDn + g.ls * (1.0 - CNDn), heat, heat_r) *
+                                                  (hyp_d - hyp), dT, 1.0 / dT);
+                        double w = quot1(1.0, 1.0 + (G < 0.0 ? 0.0 : G));
                         if (w < 0.05) w = 0.05;
                         hyp = qv + w * (hyp - qv);
                     } else {
@@ -236,7 +258,7 @@ __global__ void __launch_bounds__(256) satadj_kernel(SatArgs a, AtjupGasParams g
                 c = qv;
                 cl = qc;
                 ic = qi;
-                t_out = T / a.t_ref;
+                t_out = quot1_by(T, a.t_ref, a.t_ref_r);
                 t_dirty = true;
             }
         }
@@ -284,6 +306,10 @@ int launch_satadj(AtjupCtx* c, int gas, const AtjupGasParams& gp) {
     a.t_ref = c->P.t_ref;
     a.r_mix = c->P.r_mix;
     a.cp_mix = c->P.cp_mix;
+    a.tri = 1.0 / (gp.t_0 - gp.t_00);
+    a.kR = 1e-3 * gp.R;
+    a.kR_r = 1.0 / a.kR;
+    a.t_ref_r = 1.0 / a.t_ref;
     ATJUP_CUDA(cudaMemsetAsync(c->counters, 0, 8 * sizeof(unsigned long long), c->stream));
     const int threads = 256;
     const long long blocks = ((long long)c->NP + threads - 1) / threads;

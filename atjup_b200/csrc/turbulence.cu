@@ -16,6 +16,7 @@
 // reference runs them as separate sweeps: a cell's sources read its neighbours' clamped k*,
 // omega*, and the second clamp must not change a value a neighbour still has to read.
 #include "ctx.cuh"
+#include "quot.cuh"
 
 namespace atjup {
 namespace {
@@ -33,6 +34,7 @@ struct TurbArgs {
     const int32_t* topo;           // [jm * km]
     const float* layer_h;          // [im]
     int im, jm, km, KP, model, turb_free, turb_curv, turb_buoy, abl_taper, wall_omega;
+    double inv_2dr, inv_2dthe, inv_2dphi;   // 1 / (2 dr) and so on
     double dr, dthe, dphi, u_0, L_m, nue_max, t_ref, g, cp_mix, re_turb;
     double k_bg_free, vel_star_max, abl_height, taper_dz;
     int wall_only;                 // column_kernel: the wall law alone (the loop's wall hold)
@@ -98,14 +100,14 @@ __global__ void __launch_bounds__(128) sources_kernel(TurbArgs a) {
     double sinthe = a.sin_the[j];
     if (sinthe == 0.0) sinthe = 1.0e-5;
     const double costhe = a.geo[(size_t)i * a.jm + j].costhe;
-    const double cotanthe = costhe / sinthe;
-    const double inv_rm = 1.0 / rm;
+    const double cotanthe = quot1(costhe, sinthe);
+    const double inv_rm = quot1(1.0, rm);
     const double rmsinthe = rm * sinthe;
-    const double inv_2dr = 1.0 / (2.0 * a.dr);
-    const double inv_2dthe = 1.0 / (2.0 * a.dthe);
-    const double inv_2dphi = 1.0 / (2.0 * a.dphi);
-    const double inv_rm2dthe = inv_2dthe / rm;
-    const double inv_rmsinthe2dphi = inv_2dphi / rmsinthe;
+    const double inv_2dr = a.inv_2dr;
+    const double inv_2dthe = a.inv_2dthe;
+    const double inv_2dphi = a.inv_2dphi;
+    const double inv_rm2dthe = quot1(inv_2dthe, rm);
+    const double inv_rmsinthe2dphi = quot1(inv_2dphi, rmsinthe);
     const double *U = a.u, *V = a.v, *W = a.w;
     const double dudr = (U[cip] - U[cim]) * inv_2dr, dvdr = (V[cip] - V[cim]) * inv_2dr;
     const double dwdr = (W[cip] - W[cim]) * inv_2dr;
@@ -131,8 +133,8 @@ __global__ void __launch_bounds__(128) sources_kernel(TurbArgs a) {
     {
         const double dis_here = dmax(ds0, DIS_MIN);
         const double tke_here = dmax(tk0, 0.0);
-        cnue = (a.model == ATJUP_TURB_K_EPSILON) ? C_NUE * tke_here * tke_here / dis_here
-                                                 : tke_here / dis_here;
+        cnue = (a.model == ATJUP_TURB_K_EPSILON) ? quot1(C_NUE * tke_here * tke_here, dis_here)
+                                                 : quot1(tke_here, dis_here);
         cnue = dmin(cnue, a.nue_max);
     }
     const double u_r = a.turb_curv ? U[c] * inv_rm : 0.0;
@@ -162,42 +164,44 @@ __global__ void __launch_bounds__(128) sources_kernel(TurbArgs a) {
     if (a.model == ATJUP_TURB_K_EPSILON) {                          // Turbulence.h:886-927
         const double C_eps_1 = 1.35, C_eps_2 = 1.80;
         const double y_phys = a.turb_free ? 1.0e20 : dmax(height_m(a, i) - y_mount, L_m);
-        const double y_star = y_phys / L_m;
-        nue = C_NUE * tk0 * tk0 / dmax(ds0, DIS_MIN);
-        const double d_plus = y_phys * a.vel_star[(size_t)j * a.KP + k] / NUE_AIR;
+        const double y_star = quot1(y_phys, L_m);
+        nue = quot1(C_NUE * tk0 * tk0, dmax(ds0, DIS_MIN));
+        const double d_plus = quot1_by(y_phys * a.vel_star[(size_t)j * a.KP + k], NUE_AIR, 1.0 / NUE_AIR);
         const double f_nue = 1.0 - exp(-0.0115 * d_plus);
-        const double Re_T = tk0 * tk0 * a.u_0 * L_m / dmax(ds0 * NUE_AIR, DIS_MIN * NUE_AIR);
-        const double f_2 = 1.0 - 0.4 / 1.8 * exp(-Re_T * Re_T / 36.0);
+        const double Re_T = quot1(tk0 * tk0 * a.u_0 * L_m, dmax(ds0 * NUE_AIR, DIS_MIN * NUE_AIR));
+        const double f_2 = 1.0 - 0.4 / 1.8 * exp(quot1_by(-Re_T * Re_T, 36.0, 1.0 / 36.0));
         nue *= f_nue;
         const double y_star2 = y_star * y_star;
-        const double L_k = -2.0 * tk0 / y_star2;
-        const double L_w = -2.0 * ds0 / y_star2 * exp(-d_plus / 2.0);
+        const double L_k = quot1(-2.0 * tk0, y_star2);
+        const double L_w = quot1(-2.0 * ds0, y_star2) * exp(-d_plus / 2.0);
         const double tke_safe = dmax(tk0, DIS_MIN);
-        const double P_w = C_eps_1 * ds0 / tke_safe * prod;
-        const double Y_w = C_eps_2 * f_2 * ds0 * ds0 / tke_safe;
-        tsrc = prod - ds0 + L_k / a.re_turb;
-        dsrc = P_w - Y_w + L_w / a.re_turb;
+        const double P_w = quot1(C_eps_1 * ds0, tke_safe) * prod;
+        const double Y_w = quot1(C_eps_2 * f_2 * ds0 * ds0, tke_safe);
+        tsrc = prod - ds0 + quot1(L_k, a.re_turb);
+        dsrc = P_w - Y_w + quot1(L_w, a.re_turb);
     } else {
-        const double exp_rm_k = 1.0 / (rm + 1.0);
-        const double dtkedr_neu = nb ? (tk_ip - tk0) * (1.0 / (2.0 * a.dr)) * exp_rm_k : dtkedr;
-        const double ddisdr_neu = nb ? (ds_ip - ds0) * (1.0 / (2.0 * a.dr)) * exp_rm_k : ddisdr;
-        const double dtkedthe_neu = (tke_jp1 - tke_jm1) / (rm * 2.0 * a.dthe);
-        const double ddisdthe_neu = (dis_jp1 - dis_jm1) / (rm * 2.0 * a.dthe);
-        const double dtkedphi_neu = (tke_kp1 - tke_km1) / (rmsinthe * 2.0 * a.dphi);
-        const double ddisdphi_neu = (dis_kp1 - dis_km1) / (rmsinthe * 2.0 * a.dphi);
+        const double exp_rm_k = quot1(1.0, rm + 1.0);
+        const double d_the = rm * 2.0 * a.dthe, d_phi = rmsinthe * 2.0 * a.dphi;
+        const double r_the = rcp_of(d_the), r_phi = rcp_of(d_phi);
+        const double dtkedr_neu = nb ? (tk_ip - tk0) * a.inv_2dr * exp_rm_k : dtkedr;
+        const double ddisdr_neu = nb ? (ds_ip - ds0) * a.inv_2dr * exp_rm_k : ddisdr;
+        const double dtkedthe_neu = quot1_by(tke_jp1 - tke_jm1, d_the, r_the);
+        const double ddisdthe_neu = quot1_by(dis_jp1 - dis_jm1, d_the, r_the);
+        const double dtkedphi_neu = quot1_by(tke_kp1 - tke_km1, d_phi, r_phi);
+        const double ddisdphi_neu = quot1_by(dis_kp1 - dis_km1, d_phi, r_phi);
         const double grad_dot = dtkedr_neu * ddisdr_neu + dtkedthe_neu * ddisdthe_neu +
                                 dtkedphi_neu * ddisdphi_neu;
         if (a.model == ATJUP_TURB_K_OMEGA) {                        // Turbulence.h:930-1017
             const double bet_star = 0.09, gam = 0.52, C_lim = 0.875, bet_0 = 0.0708;
-            const double dudr_k = (U[cip] - U[cim]) / (2.0 * a.dr) / (rm + 1.0);
-            const double dvdthe_k = (V[cjp] - V[cjm]) / (rm * 2.0 * a.dthe);
-            const double dwdphi_k = (W[ckp] - W[ckm]) / (rmsinthe * 2.0 * a.dphi);
-            const double dudthe_u = (U[cjp] - U[cjm]) / (rm * 2.0 * a.dthe);
-            const double dudphi_u = (U[ckp] - U[ckm]) / (rmsinthe * 2.0 * a.dphi);
-            const double dvdr_u = (V[cip] - V[cim]) / (2.0 * a.dr) / (rm + 1.0);
-            const double dwdr_u = (W[cip] - W[cim]) / (2.0 * a.dr) / (rm + 1.0);
-            const double dvdphi_u = (V[ckp] - V[ckm]) / (rmsinthe * 2.0 * a.dphi);
-            const double dwdthe_u = (W[cjp] - W[cjm]) / (rm * 2.0 * a.dthe);
+            const double dudr_k = quot1(quot1(U[cip] - U[cim], 2.0 * a.dr), rm + 1.0);
+            const double dvdthe_k = quot1_by(V[cjp] - V[cjm], d_the, r_the);
+            const double dwdphi_k = quot1_by(W[ckp] - W[ckm], d_phi, r_phi);
+            const double dudthe_u = quot1_by(U[cjp] - U[cjm], d_the, r_the);
+            const double dudphi_u = quot1_by(U[ckp] - U[ckm], d_phi, r_phi);
+            const double dvdr_u = quot1(quot1(V[cip] - V[cim], 2.0 * a.dr), rm + 1.0);
+            const double dwdr_u = quot1(quot1(W[cip] - W[cim], 2.0 * a.dr), rm + 1.0);
+            const double dvdphi_u = quot1_by(V[ckp] - V[ckm], d_phi, r_phi);
+            const double dwdthe_u = quot1_by(W[cjp] - W[cjm], d_the, r_the);
             const double S11 = dudr_k, S22 = dvdthe_k, S33 = dwdphi_k;
             const double S12 = 0.5 * (dudthe_u + dvdr_u);
             const double S13 = 0.5 * (dudphi_u + dwdr_u);
@@ -208,40 +212,44 @@ __global__ void __launch_bounds__(128) sources_kernel(TurbArgs a) {
             const double sig_d = (grad_dot <= 0.0) ? 0.0 : 0.125;
             const double bd = bet_star * dmax(ds0, 1.0e-20);
             const double chi_w = fabs(Omega * Omega * S_mag / (bd * bd * bd));   // pow(bd, 3)
-            const double f_bet = (1.0 + 85.0 * chi_w) / (1.0 + 100.0 * chi_w);
+            const double f_bet = quot1(1.0 + 85.0 * chi_w, 1.0 + 100.0 * chi_w);
             const double bet_wc = bet_0 * f_bet;
-            nue = tk0 / dmax(w_hat, 1.0e-20);
+            nue = quot1(tk0, dmax(w_hat, 1.0e-20));
             const double P_k = dmin(prod, 20.0 * bet_star * tk0 * ds0);
             const double Y_k = bet_star * tk0 * ds0;
-            const double P_w = gam * ds0 / dmax(tk0, 1.0e-20) * P_k;
+            const double P_w = quot1(gam * ds0, dmax(tk0, 1.0e-20)) * P_k;
             const double Y_w = bet_wc * ds0 * ds0;
-            const double D_w = sig_d / dmax(ds0, 1.0e-20) * grad_dot;
+            const double D_w = quot1(sig_d, dmax(ds0, 1.0e-20)) * grad_dot;
             tsrc = P_k - Y_k;
             dsrc = P_w - Y_w + D_w;
         } else {                                                    // Turbulence.h:1021-1106
             const double a1 = 0.31, bet_star = 0.09, bet1 = 0.0333, bet2 = 0.0368;
             const double gam1 = 0.413, gam2 = 0.2, sig_w2 = 1.168;
-            const double nue_air_nd = NUE_AIR / (a.u_0 * L_m);
+            const double nue_air_nd = quot1(NUE_AIR, a.u_0 * L_m);
             const double dz_layer = dmax(1.0, layer_dz_m(a, i - 1 > 0 ? i - 1 : 0));
             const double y_phys = a.turb_free ? 1.0e20 : dmax(height_m(a, i) - y_mount, dz_layer);
-            const double y_star = y_phys / L_m;
-            const double CD_kw = dmax(2.0 * sig_w2 / dmax(ds0, 1.0e-20) * grad_dot, 1.0e-20);
+            const double y_star = quot1(y_phys, L_m);
             const double dis_safe = dmax(ds0, 1.0e-20);
-            const double arg1 = dmin(dmax(sqrt(tk0) / (bet_star * dis_safe * y_star),
-                                          500.0 * nue_air_nd / (y_star * y_star * dis_safe)),
-                                     4.0 * sig_w2 * tk0 / (CD_kw * y_star * y_star));
-            const double arg2 = dmax(2.0 * sqrt(tk0) / (bet_star * dis_safe * y_star),
-                                     500.0 * nue_air_nd / (y_star * y_star * dis_safe));
+            const double sw = quot1(2.0 * sig_w2, dis_safe);
+            const double CD_kw = dmax(sw * grad_dot, 1.0e-20);
+            const double s_tk = sqrt(tk0);
+            const double num[4] = {s_tk, 500.0 * nue_air_nd, 4.0 * sig_w2 * tk0, 2.0 * s_tk};
+            const double den[4] = {bet_star * dis_safe * y_star, y_star * y_star * dis_safe, CD_kw * y_star * y_star,
+                                   bet_star * dis_safe * y_star};
+            double arg[4];
+            quots(num, den, arg);
+            const double arg1 = dmin(dmax(arg[0], arg[1]), arg[2]);
+            const double arg2 = dmax(arg[3], arg[1]);
             const double a1sq = arg1 * arg1;
             const double F1 = tanh(a1sq * a1sq);                                // pow(arg1, 4)
             const double F2 = tanh(arg2 * arg2);                                // pow(arg2, 2)
-            nue = a1 * tk0 / dmax(a1 * dis_safe, Omega * F2);
+            nue = quot1(a1 * tk0, dmax(a1 * dis_safe, Omega * F2));
             const double tke_safe = dmax(tk0, 1.0e-20);
             const double P_k = dmin(prod, 20.0 * bet_star * tke_safe * dis_safe);
             const double Y_k = bet_star * tke_safe * dis_safe;
-            const double P_w = (F1 * gam1 + (1.0 - F1) * gam2) * P_k * dis_safe / tke_safe;
+            const double P_w = quot1((F1 * gam1 + (1.0 - F1) * gam2) * P_k * dis_safe, tke_safe);
             const double Y_w = (F1 * bet1 + (1.0 - F1) * bet2) * dis_safe * dis_safe;
-            const double D_w = 2.0 * (1.0 - F1) * sig_w2 / dis_safe * grad_dot;
+            const double D_w = quot1(2.0 * (1.0 - F1) * sig_w2, dis_safe) * grad_dot;
             tsrc = P_k - Y_k;
             dsrc = P_w - Y_w + D_w;
         }
@@ -249,12 +257,12 @@ __global__ void __launch_bounds__(128) sources_kernel(TurbArgs a) {
     if (a.turb_buoy != 0) {                                         // Turbulence.h:843-867
         const double T = a.t[c] * a.t_ref;
         const double dz = height_m(a, i + 1) - height_m(a, i - 1);
-        const double dTdz = (a.t[cip] - a.t[cim]) * a.t_ref / dz;
-        const double Gam = a.g / a.cp_mix;
-        const double N2 = (T > 0.0 && dz > 0.0) ? a.g / T * (dTdz + Gam) * 1.0 : 0.0;
+        const double dTdz = quot1((a.t[cip] - a.t[cim]) * a.t_ref, dz);
+        const double Gam = quot1(a.g, a.cp_mix);
+        const double N2 = (T > 0.0 && dz > 0.0) ? quot1(a.g, T) * (dTdz + Gam) * 1.0 : 0.0;
         if (isfinite(N2) && (N2 > 0.0 || a.turb_buoy == 2)) {
-            const double tL = L_m / a.u_0;
-            tsrc -= dmax(0.0, nue) * N2 * tL * tL / 0.9;
+            const double tL = quot1(L_m, a.u_0);
+            tsrc -= quot1_by(dmax(0.0, nue) * N2 * tL * tL, 0.9, 1.0 / 0.9);
         }
     }
     a.prod[c] = prod;
@@ -437,6 +445,7 @@ TurbArgs turb_args(AtjupCtx* c) {
     a.im = P.im; a.jm = P.jm; a.km = P.km; a.KP = c->KP;
     a.model = H.turb_model; a.turb_free = H.turb_free; a.turb_curv = H.turb_curv;
     a.turb_buoy = H.turb_buoy; a.abl_taper = H.abl_taper; a.wall_omega = H.turb_wall_omega;
+    a.inv_2dr = 1.0 / (2.0 * P.dr); a.inv_2dthe = 1.0 / (2.0 * P.dthe); a.inv_2dphi = 1.0 / (2.0 * P.dphi);
     a.dr = P.dr; a.dthe = P.dthe; a.dphi = P.dphi; a.u_0 = P.u_0;
     a.L_m = P.L_atm * 1.0e3;
     a.nue_max = H.nue_max_phys / (P.u_0 * a.L_m);

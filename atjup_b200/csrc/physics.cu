@@ -49,12 +49,11 @@ struct PhysStage {
     double *prod, *tke_source, *dis_source;
     const uint8_t* flags;
     const GeoIJ* geo;
-    int im, jm, km, KP, stage;
-    // FP64 step: the species keep no accumulator. Stage s's right-hand side is recovered from the
+    int im, jm, km, KP;
+    // FP64 step (acc_free): the species keep no accumulator. Stage s's right-hand side is recovered from the
     // next stage input as (X_{s+1} - y_n) / c_s (exact: X_{s+1} lies within a factor 2 of y_n,
     // so the subtraction is exact, Sterbenz), so stage 3 reads X1 and X2 beside its own input X3
     // instead of one accumulator that stages 0-2 would each write and stages 1-2 read.
-    int acc_free;
     const double* x1[ATJUP_S_COUNT];   // X1, X2 of the species (stage 3, acc_free)
     const double* x2[ATJUP_S_COUNT];
     double inv_c_half, inv_dt;         // 1 / c of stages 0 and 1 (2 / dt) and of stage 2 (1 / dt)
@@ -87,14 +86,14 @@ __device__ __forceinline__ double layer_dz_m(const PhysStage& a, int i) {
 }
 
 struct Cell {
-    size_t c, cip, cim, cjp, cjm, ckp, ckm;
+    unsigned c, cip, cim, cjp, cjm, ckp, ckm;      // a field has fewer than 2^32 cells
 };
 
 // The cell and its six neighbours; the i and j neighbours of the block's faces are clamped to the
 // cell itself (those cells are never integrated: their loads only have to stay in bounds).
 __device__ __forceinline__ Cell cell_of(const PhysStage& a, int i, int j, int k) {
     Cell x;
-    const size_t row = ((size_t)i * a.jm + j) * a.KP, plane = (size_t)a.jm * a.KP;
+    const unsigned row = ((unsigned)i * a.jm + j) * a.KP, plane = (unsigned)a.jm * a.KP;
     const int ke = (k >= a.km - 2) ? 0 : k + 1, kw = (k == 0) ? a.km - 2 : k - 1;
     x.c = row + k;
     x.cip = (i < a.im - 1) ? x.c + plane : x.c;
@@ -109,11 +108,11 @@ __device__ __forceinline__ Cell cell_of(const PhysStage& a, int i, int j, int k)
 // RK bookkeeping of one scalar at an integrated cell (RungeKutta_Jup_Turb.cpp:425-490, 493-568).
 // The accumulator is summed in R and stored as TA; the next stage input and the final update are
 // formed in FP64 from the FP64 time-level-n value, then clamped, then stored as TO.
-template <typename TO, typename TA, typename R>
+template <int ST, typename TO, typename TA, typename R>
 __device__ __forceinline__ void rk_update(const PhysStage& a, int s, size_t c, R rhs, R acc_in,
                                           double qn) {
-    const R acc = (a.stage == 0) ? (R)a.wgt * rhs : acc_in + (R)a.wgt * rhs;
-    if (a.stage < 3) {
+    const R acc = (ST == 0) ? (R)a.wgt * rhs : acc_in + (R)a.wgt * rhs;
+    if (ST < 3) {
         static_cast<TA*>(a.acc[s])[c] = (TA)acc;
         double x = qn + (double)((R)a.c_in * rhs);
         if (s == ATJUP_S_COUNT) x = safe_clamp(x, 0.0, a.tke_max_nd);          // k*
@@ -150,6 +149,16 @@ __device__ __forceinline__ int precip_slot(int s) {
 // step keeps FP32 stage buffers and accumulators and FP32 arithmetic: stage 0 <double, float,
 // float, float> (it reads the live fields), stages 1-2 <float, float, float, float>, stage 3
 // <float, double, float, float>.
+
+template <typename R> constexpr bool acc_free = sizeof(R) == 8;
+// Block shape and blocks per SM of the two stage kernels, which wait for memory: the more warps the better, until
+// the registers spill. Blocks of 128 threads, as a block's slot is held until its last warp ends and some
+// warps leave at once (solid cells, the rows by the poles). With the stage a template argument the species
+// fit 72 registers. 41x181x361, us a stage: 256 threads at 80 registers 282, 128 threads 265, then by stage 233
+// at 80 registers, 224 at 72, 232 at 64; mixed (stages 0, 1, 3) 354, 265, 216 before, 222, 202, 179 at 64 and 217, 199,
+// 174 at 56. Closure 129 before, 134, 131, 123 at 80, 72, 64 and mixed 111, 100, 96.
+constexpr int PS_K = 64, PS_J = 2, CL_BLOCKS = 8;
+template <typename R> constexpr int SP_BLOCKS = sizeof(R) == 8 ? 7 : 9;
 
 // One thread per cell, the eleven species in turn (an unrolled loop: each species' index, sources
 // and coefficients are compile-time): what the species share -- the cell's indices, its flags,
@@ -195,10 +204,10 @@ __device__ __forceinline__ R species_rhs(const PhysStage& a, const CellShared<R>
 
 // FP64 step, no accumulator: the next stage input, or at stage 3 the clamped result from the
 // right-hand sides recovered from X1, X2, X3 (f0)
-template <int S>
+template <int S, int ST>
 __device__ __forceinline__ double species_acc_free_out(const PhysStage& a, double r, double f0,
                                                        double qn, double x1, double x2) {
-    if (a.stage < 3) return qn + a.c_in * r;
+    if (ST < 3) return qn + a.c_in * r;
     const double k1 = (x1 - qn) * a.inv_c_half, k2 = (x2 - qn) * a.inv_c_half;
     const double k3 = (f0 - qn) * a.inv_dt;
     const double acc = ((k1 + 2.0 * k2) + 2.0 * k3) + r;
@@ -229,7 +238,7 @@ struct SpIn {
     double qn, x1, x2, src0, src1;
 };
 
-template <int S, typename TI, typename TA, typename R>
+template <int S, int ST, typename TI, typename TA, typename R>
 __device__ __forceinline__ SpIn<R> species_load(const PhysStage& a, const Cell& x) {
     SpIn<R> v;
     const size_t c = x.c;
@@ -240,9 +249,9 @@ __device__ __forceinline__ SpIn<R> species_load(const PhysStage& a, const Cell& 
     v.acc_in = (R)0;
     v.x1 = 0.0;
     v.x2 = 0.0;
-    if (a.acc_free) {
-        if (a.stage == 3) { v.x1 = a.x1[S][c]; v.x2 = a.x2[S][c]; }
-    } else if (a.stage > 0) {
+    if constexpr (acc_free<R>) {
+        if (ST == 3) { v.x1 = a.x1[S][c]; v.x2 = a.x2[S][c]; }
+    } else if (ST > 0) {
         v.acc_in = (R)static_cast<const TA*>(a.acc[S])[c];
     }
     const double* s1 = species_src1<S>(a);
@@ -251,35 +260,32 @@ __device__ __forceinline__ SpIn<R> species_load(const PhysStage& a, const Cell& 
     return v;
 }
 
-template <int S, typename TO, typename TA, typename R>
+template <int S, int ST, typename TO, typename TA, typename R>
 __device__ __forceinline__ void species_finish(const PhysStage& a, size_t c, const CellShared<R>& z,
                                                const SpIn<R>& v) {
     const R r = species_rhs<S, R>(a, z, v.f0, v.fip, v.fim, v.fjp, v.fjm, v.fkp, v.fkm, v.src0, v.src1);
-    if (a.acc_free) {
-        static_cast<TO*>(a.q_out[S])[c] =
-            (TO)species_acc_free_out<S>(a, (double)r, (double)v.f0, v.qn, v.x1, v.x2);
-        return;
-    }
-    rk_update<TO, TA, R>(a, S, c, r, v.acc_in, v.qn);
+    if constexpr (acc_free<R>)
+        static_cast<TO*>(a.q_out[S])[c] = (TO)species_acc_free_out<S, ST>(a, (double)r, (double)v.f0, v.qn, v.x1, v.x2);
+    else
+        rk_update<ST, TO, TA, R>(a, S, c, r, v.acc_in, v.qn);
 }
 
-template <int S, typename TI, typename TO, typename TA, typename R>
+template <int S, int ST, typename TI, typename TO, typename TA, typename R>
 __device__ __forceinline__ void species_all(const PhysStage& a, const Cell& x,
                                             const CellShared<R>& z, const SpIn<R>& cur) {
     if constexpr (S + 1 < ATJUP_S_COUNT) {
-        const SpIn<R> nxt = species_load<S + 1, TI, TA, R>(a, x);
-        species_finish<S, TO, TA, R>(a, x.c, z, cur);
-        species_all<S + 1, TI, TO, TA, R>(a, x, z, nxt);
+        const SpIn<R> nxt = species_load<S + 1, ST, TI, TA, R>(a, x);
+        species_finish<S, ST, TO, TA, R>(a, x.c, z, cur);
+        species_all<S + 1, ST, TI, TO, TA, R>(a, x, z, nxt);
     } else {
-        species_finish<S, TO, TA, R>(a, x.c, z, cur);
+        species_finish<S, ST, TO, TA, R>(a, x.c, z, cur);
     }
 }
 
-// Three blocks per SM (at most 80 registers): with two species' loads in flight the FP64 form
-// needs 96 registers unbounded (two blocks per SM) and spills heavily at 64 (four blocks); the
-// step measured 6.77 ms at 80 against 7.06 at 96, 7.14 at 64 and 6.89 without the early loads.
-template <typename TI, typename TO, typename TA, typename R>
-__global__ void __launch_bounds__(256, 3) species_stage_kernel(PhysStage a) {
+// Bound by memory latency: about 440 bytes a cell, 4.3 TB/s at 282 us. (Species shared out over blocks: slower,
+// 319 us in two groups, 393 in four, as each group reads the shared fields again.)
+template <int ST, typename TI, typename TO, typename TA, typename R>
+__global__ void __launch_bounds__(PS_K * PS_J, SP_BLOCKS<R>) species_stage_kernel(PhysStage a) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int i = blockIdx.z;
@@ -295,7 +301,7 @@ __global__ void __launch_bounds__(256, 3) species_stage_kernel(PhysStage a) {
     const double rho = a.rho_mix[c];
     if (!(fl & NB_INT)) {
         // the cell keeps its live values through the step
-        if (a.stage < 3) {
+        if (ST < 3) {
 #pragma unroll
             for (int s = 0; s < ATJUP_S_COUNT; s++)
                 static_cast<TO*>(a.q_out[s])[c] = (TO)a.q_live[s][c];
@@ -327,28 +333,26 @@ __global__ void __launch_bounds__(256, 3) species_stage_kernel(PhysStage a) {
         z.nue_t_s = (R)nue_t64 / (R)0.9;
         z.fall = (R)(a.stokes_pre * (a.rg_nh4sh - rho) * a.g / a.mue_mix / a.u_0);
     }
-    species_all<0, TI, TO, TA, R>(a, x, z, species_load<0, TI, TA, R>(a, x));
+    species_all<0, ST, TI, TO, TA, R>(a, x, z, species_load<0, ST, TI, TA, R>(a, x));
 }
 
 // k*, omega*: transport, diffusion with the model's coefficients, and the closure sources
 // (RHS_Jup_Turb.cpp:257-303, 736-998, 1399-1452). One instantiation per closure model, so that
-// each holds the registers of its own branch only. Three blocks per SM (at most 80 registers: the
-// k-omega SST form spilled 172 bytes at 64; the step measured 6.70 ms against 6.72 at 64 and 6.82
-// at 128).
-template <int MODEL, typename TI, typename TO, typename TA, typename R>
-__global__ void __launch_bounds__(256, 3) closure_stage_kernel(PhysStage a) {
+// each holds the registers of its own branch only.
+template <int MODEL, int ST, typename TI, typename TO, typename TA, typename R>
+__global__ void __launch_bounds__(PS_K * PS_J, CL_BLOCKS) closure_stage_kernel(PhysStage a) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int i = blockIdx.z;
     if (k >= a.km || j >= a.jm) return;
-    const int ST = ATJUP_S_COUNT, SD = ATJUP_S_COUNT + 1;
+    const int QT = ATJUP_S_COUNT, QD = ATJUP_S_COUNT + 1;
     // Every load is issued before the integrated-cell test (one memory round trip): the
     // neighbour addresses are clamped into the block, so boundary cells read only their own
     // cell before the test sends them to the copy below.
     const Cell x = cell_of(a, i, j, k);
     const uint8_t fl = a.flags[x.c];
-    const TI* TK = static_cast<const TI*>(a.q_in[ST]);
-    const TI* DS = static_cast<const TI*>(a.q_in[SD]);
+    const TI* TK = static_cast<const TI*>(a.q_in[QT]);
+    const TI* DS = static_cast<const TI*>(a.q_in[QD]);
     const TI* Us = static_cast<const TI*>(a.u);
     const TI* Vs = static_cast<const TI*>(a.v);
     const TI* Ws = static_cast<const TI*>(a.w);
@@ -367,9 +371,9 @@ __global__ void __launch_bounds__(256, 3) closure_stage_kernel(PhysStage a) {
     const double nv = a.nue[x.c];
     const int32_t topo = a.topo[(size_t)j * a.km + k];
     if (!(fl & NB_INT)) {
-        if (a.stage < 3) {
-            static_cast<TO*>(a.q_out[ST])[x.c] = (TO)a.q_live[ST][x.c];
-            static_cast<TO*>(a.q_out[SD])[x.c] = (TO)a.q_live[SD][x.c];
+        if (ST < 3) {
+            static_cast<TO*>(a.q_out[QT])[x.c] = (TO)a.q_live[QT][x.c];
+            static_cast<TO*>(a.q_out[QD])[x.c] = (TO)a.q_live[QD][x.c];
         }
         return;
     }
@@ -591,19 +595,19 @@ __global__ void __launch_bounds__(256, 3) closure_stage_kernel(PhysStage a) {
     if (!isfinite(dis_src)) dis_src = (R)0;
     tke_src = dmax(-tke_src_max, dmin(tke_src_max, tke_src));
     dis_src = dmax(-dis_src_max, dmin(dis_src_max, dis_src));
-    if (a.stage == 3) {
+    if (ST == 3) {
         a.prod[x.c] = (double)P_full;
         a.tke_source[x.c] = (double)tke_src;
         a.dis_source[x.c] = (double)dis_src;
     }
     // the accumulators and n copies are read here, not with the stencil: read early they hold
     // four more registers (8 in FP64) through the whole source computation
-    const R acc_t = (a.stage == 0) ? (R)0 : (R)static_cast<const TA*>(a.acc[ST])[x.c];
-    const R acc_d = (a.stage == 0) ? (R)0 : (R)static_cast<const TA*>(a.acc[SD])[x.c];
-    rk_update<TO, TA, R>(a, ST, x.c, -transport_tke + diffusion_tke * dtre + tke_src, acc_t,
-                         a.q_n[ST][x.c]);
-    rk_update<TO, TA, R>(a, SD, x.c, -transport_dis + diffusion_dis * ddre + dis_src, acc_d,
-                         a.q_n[SD][x.c]);
+    const R acc_t = (ST == 0) ? (R)0 : (R)static_cast<const TA*>(a.acc[QT])[x.c];
+    const R acc_d = (ST == 0) ? (R)0 : (R)static_cast<const TA*>(a.acc[QD])[x.c];
+    rk_update<ST, TO, TA, R>(a, QT, x.c, -transport_tke + diffusion_tke * dtre + tke_src, acc_t,
+                         a.q_n[QT][x.c]);
+    rk_update<ST, TO, TA, R>(a, QD, x.c, -transport_dis + diffusion_dis * ddre + dis_src, acc_d,
+                         a.q_n[QD][x.c]);
 }
 
 }  // namespace
@@ -659,8 +663,7 @@ PhysStage stage_args(AtjupCtx* c, int stage, const void* const* vin) {
     a.dis_source = c->f[ATJUP_F_DIS_SOURCE];
     a.flags = c->nbflags;
     a.geo = c->geo;
-    a.im = P.im; a.jm = P.jm; a.km = P.km; a.KP = c->KP; a.stage = stage;
-    a.acc_free = (c->step_prec != ATJUP_PREC_MIXED) ? 1 : 0;
+    a.im = P.im; a.jm = P.jm; a.km = P.km; a.KP = c->KP;
     a.inv_c_half = 2.0 / P.dt;
     a.inv_dt = 1.0 / P.dt;
     a.c_in = (stage == 0 || stage == 1) ? 0.5 * P.dt : (stage == 2 ? P.dt : 0.0);
@@ -699,25 +702,25 @@ PhysStage stage_args(AtjupCtx* c, int stage, const void* const* vin) {
 }
 }  // namespace
 
-template <typename TI, typename TO, typename TA, typename R>
+template <int ST, typename TI, typename TO, typename TA, typename R>
 static int launch_typed(AtjupCtx* c, const PhysStage& a, int what, cudaStream_t st) {
     const AtjupParams& P = c->P;
-    const dim3 block(128, 2);
-    const dim3 grid((P.km + 127) / 128, (P.jm + 1) / 2, P.im);
+    const dim3 block(PS_K, PS_J);
+    const dim3 grid((P.km + PS_K - 1) / PS_K, (P.jm + PS_J - 1) / PS_J, P.im);
     if (what == 0) {
-        species_stage_kernel<TI, TO, TA, R><<<grid, block, 0, st>>>(a);
+        species_stage_kernel<ST, TI, TO, TA, R><<<grid, block, 0, st>>>(a);
         c->launches++;
         ATJUP_CHECK_LAUNCH("species_stage_kernel");
     } else {
         switch (a.turb_model) {
         case ATJUP_TURB_K_EPSILON:
-            closure_stage_kernel<ATJUP_TURB_K_EPSILON, TI, TO, TA, R><<<grid, block, 0, st>>>(a);
+            closure_stage_kernel<ATJUP_TURB_K_EPSILON, ST, TI, TO, TA, R><<<grid, block, 0, st>>>(a);
             break;
         case ATJUP_TURB_K_OMEGA:
-            closure_stage_kernel<ATJUP_TURB_K_OMEGA, TI, TO, TA, R><<<grid, block, 0, st>>>(a);
+            closure_stage_kernel<ATJUP_TURB_K_OMEGA, ST, TI, TO, TA, R><<<grid, block, 0, st>>>(a);
             break;
         default:
-            closure_stage_kernel<ATJUP_TURB_K_OMEGA_SST, TI, TO, TA, R><<<grid, block, 0, st>>>(a);
+            closure_stage_kernel<ATJUP_TURB_K_OMEGA_SST, ST, TI, TO, TA, R><<<grid, block, 0, st>>>(a);
         }
         c->launches++;
         ATJUP_CHECK_LAUNCH("closure_stage_kernel");
@@ -730,10 +733,15 @@ static int launch_typed(AtjupCtx* c, const PhysStage& a, int what, cudaStream_t 
 // buffers)
 int launch_phys_stage(AtjupCtx* c, int stage, const void* const* vin, int what, cudaStream_t st) {
     const PhysStage a = stage_args(c, stage, vin);
-    if (c->step_prec != ATJUP_PREC_MIXED) return launch_typed<double, double, double, double>(c, a, what, st);
-    if (stage == 0) return launch_typed<double, float, float, float>(c, a, what, st);
-    if (stage < 3) return launch_typed<float, float, float, float>(c, a, what, st);
-    return launch_typed<float, double, float, float>(c, a, what, st);
+    // (the bookkeeping of stages 1 and 2 is the same)
+    if (c->step_prec != ATJUP_PREC_MIXED) {
+        if (stage == 0) return launch_typed<0, double, double, double, double>(c, a, what, st);
+        if (stage < 3) return launch_typed<1, double, double, double, double>(c, a, what, st);
+        return launch_typed<3, double, double, double, double>(c, a, what, st);
+    }
+    if (stage == 0) return launch_typed<0, double, float, float, float>(c, a, what, st);
+    if (stage < 3) return launch_typed<1, float, float, float, float>(c, a, what, st);
+    return launch_typed<3, float, double, float, float>(c, a, what, st);
 }
 
 }  // namespace atjup

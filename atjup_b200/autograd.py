@@ -57,16 +57,18 @@ class IterationStep(torch.autograd.Function):
     def forward(ctx, model, iter_n, first, chained, *x):
         from .params import LIN_FIELDS
         y = tuple(t.detach().contiguous() for t in x)
-        if not chained:
-            # chained: x are the outputs of the step just run, which the context still holds
-            model.set_state_tensors(y, names=LIN_FIELDS, wait=False)
         stages = [torch.empty_like(y[0]) for _ in range(12)]
-        model.set_stage_buffers(stages)
-        try:
-            model.step(iter_n, first)
-        finally:
-            model.set_stage_buffers(None)
-        out = model.state_tensors(LIN_FIELDS)
+        out = [torch.empty_like(y[0]) for _ in LIN_FIELDS]
+        with model.ordered(*y):
+            if not chained:
+                # chained: x are the outputs of the step just run, which the context still holds
+                model.copy_fields(y, LIN_FIELDS, True)
+            model.stage_buffers(stages)
+            try:
+                model.step(iter_n, first)
+            finally:
+                model.stage_buffers(None)
+            model.copy_fields(out, LIN_FIELDS, False)
         ctx.model, ctx.iter_n, ctx.first = model, iter_n, first
         ctx.save_for_backward(*y, *stages)
         return tuple(out)
@@ -77,10 +79,11 @@ class IterationStep(torch.autograd.Function):
         saved = ctx.saved_tensors
         y, stages = saved[:len(LIN_FIELDS)], saved[len(LIN_FIELDS):]
         model = ctx.model
-        model.set_state_tensors(y, names=LIN_FIELDS, wait=False)   # the linearisation point
         g = [torch.zeros_like(r) if gr is None else gr.detach().clone().contiguous()
              for gr, r in zip(grads, y)]
-        model.iteration_adjoint_ckpt(g, stages, ctx.iter_n, ctx.first)
+        with model.ordered(*y, *stages):
+            model.copy_fields(y, LIN_FIELDS, True)      # the linearisation point
+            model.queue_iteration_adjoint(g, stages, ctx.iter_n, ctx.first)
         return (None, None, None, None, *g)
 
 

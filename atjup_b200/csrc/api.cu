@@ -325,25 +325,24 @@ int atjup_gpu_set_grid(AtjupCtx* c, const double* rad, const double* the, const 
     // per-cell flags for the RK stage: bit 0 solid, 1..6 solid neighbour (i+1, i-1, j+1, j-1,
     // k+1 and k-1 on the meridian ring), 7 integrated by the RK step
     std::vector<uint8_t> nbh(c->NP, 0);
+    const std::vector<uint8_t> open_row(KP, 0);             // beyond the grid: not solid
     for (int i = 0; i < im; i++)
-        for (int j = 0; j < jm; j++)
-            for (int k = 0; k < km; k++) {
-                auto S_ = [&](int ii, int jj, int kk) -> bool {
-                    if (ii < 0 || ii >= im || jj < 0 || jj >= jm || kk < 0 || kk >= km) return false;
-                    return solid[((size_t)ii * jm + jj) * km + kk] != 0;
-                };
-                const int ke = (k >= km - 2) ? 0 : k + 1, kw = (k == 0) ? km - 2 : k - 1;
-                uint8_t f = 0;
-                if (S_(i, j, k)) f |= 1;
-                if (S_(i + 1, j, k)) f |= 2;
-                if (S_(i - 1, j, k)) f |= 4;
-                if (S_(i, j + 1, k)) f |= 8;
-                if (S_(i, j - 1, k)) f |= 16;
-                if (S_(i, j, ke)) f |= 32;
-                if (S_(i, j, kw)) f |= 64;
-                if (i >= 1 && i <= im - 2 && j >= 3 && j <= jm - 4 && k <= km - 2 && !(f & 1)) f |= 128;
-                nbh[((size_t)i * jm + j) * KP + k] = f;
-            }
+        for (int j = 0; j < jm; j++) {
+            const size_t r = ((size_t)i * jm + j) * KP, pl = (size_t)jm * KP;
+            const uint8_t* s = &s_pad[r];
+            const uint8_t* ip = i + 1 < im ? s + pl : open_row.data();
+            const uint8_t* in = i > 0 ? s - pl : open_row.data();
+            const uint8_t* jp = j + 1 < jm ? s + KP : open_row.data();
+            const uint8_t* jn = j > 0 ? s - KP : open_row.data();
+            const bool inner = i >= 1 && i <= im - 2 && j >= 3 && j <= jm - 4;
+            auto flags = [&](int k, int ke, int kw) {
+                const uint8_t own = inner && k <= km - 2 && !s[k] ? 128 : 0;
+                return (uint8_t)(s[k] | ip[k] << 1 | in[k] << 2 | jp[k] << 3 | jn[k] << 4 | s[ke] << 5 | s[kw] << 6 | own);
+            };
+            nbh[r] = flags(0, 1, km - 2);
+            for (int k = 1; k < km - 2; k++) nbh[r + k] = flags(k, k + 1, k - 1);
+            for (int k = km - 2; k < km; k++) nbh[r + k] = flags(k, 0, k - 1);
+        }
     // solid-cell list for bcSolidGround (BC_Jup.h:496-590): first direction with two fluid cells
     auto sol = [&](int i, int j, int k) -> bool {
         if (i < 0 || i >= im || j < 0 || j >= jm || k < 0 || k >= km) return true;
@@ -358,8 +357,9 @@ int atjup_gpu_set_grid(AtjupCtx* c, const double* rad, const double* the, const 
     for (int i = 0; i < im; i++)
         for (int j = 0; j < jm; j++) {
             bool any = false;
+            const uint8_t* srow = solid + ((size_t)i * jm + j) * km;
             for (int k = 0; k < km; k++) {
-                if (!sol(i, j, k)) continue;
+                if (!srow[k]) continue;
                 any = true;
                 SolidCell sc{};
                 sc.c = (int64_t)(((size_t)i * jm + j) * KP + k);

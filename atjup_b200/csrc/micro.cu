@@ -7,7 +7,7 @@
 //   difflux_kernel        the diffusive fluxes of DiffMassFluxJup (ChemistryJup.h:375-538, 756-780)
 //   massflux_kernel       ChemMassRateJup: reaction rate + diffusive flux (ChemistryJup.h:59-281)
 //   fluxlim_kernel        FluxLimiter<cJupiterModel>::nh4sh (FluxLimiter.h)
-//   clamp_species_kernel  clampNegativeSpecies (FileIO_Jup.cpp:494-548)
+//   sync_n_kernel         clampNegativeSpecies (FileIO_Jup.cpp:494-548)
 //   diagnostics_kernel    cJupiterModel::Forces (InitValues_Jup.cpp:742-812) and Latent_Heat
 //                         (Thermo_Jup.cpp:89-232): output fields only
 //
@@ -553,17 +553,11 @@ __global__ void fluxlim_kernel(MicroArgs a) {
     a.fluxlim[c] = corr;
 }
 
-__global__ void clamp_species_kernel(MicroArgs a) {
-    int i, j, k;
-    size_t c;
-    if (!cell_index(a, i, j, k, c)) return;
-    for (int s = 0; s < ATJUP_S_COUNT; s++)
-        if (!(a.q[s][c] >= 0.0)) a.q[s][c] = 0.0;
-}
-
 // live -> time-level-n copies of a list of transported scalars, the negative (or NaN) values of the
-// first n_clamp of them set to 0 in both (clampNegativeSpecies). One pass over the fields in place of a
-// pass that clamps and a copy per field; bound by memory (16 B per cell and field).
+// first n_clamp of them set to 0 in both (clampNegativeSpecies); without time-level-n fields the clamp alone. One
+// pass over the fields in place of a pass that clamps and a copy per field, a field per blockIdx.y; bound by
+// memory (16 B per cell and field, the clamp alone 8: 41x181x361 60 us with a thread per cell taking the fields in
+// turn, 39 so).
 struct SyncArgs {
     double* live[ATJUP_S_COUNT + 2];
     double* n[ATJUP_S_COUNT + 2];
@@ -583,6 +577,7 @@ __global__ void __launch_bounds__(256) sync_n_kernel(const __grid_constant__ Syn
         if (!(v1.x >= 0.0)) x[c + 2] = v1.x = 0.0;
         if (!(v1.y >= 0.0)) x[c + 3] = v1.y = 0.0;
     }
+    if (!y) return;
     *reinterpret_cast<double2*>(y + c) = v0;
     *reinterpret_cast<double2*>(y + c + 2) = v1;
 }
@@ -810,10 +805,15 @@ int launch_micro(AtjupCtx* c, int what) {
         if ((rc = launch_shapiro(c, a.fluxlim, 2, 1.0, 1, 1))) return rc;
         break;
     }
-    case MICRO_CLAMP:
-        clamp_species_kernel<<<gcell, TB, 0, c->stream>>>(a);
+    case MICRO_CLAMP: {
+        SyncArgs s{};
+        for (int q = 0; q < ATJUP_S_COUNT; q++) s.live[q] = a.q[q];
+        s.n_clamp = ATJUP_S_COUNT;
+        s.N = c->NP;
+        sync_n_kernel<<<dim3((unsigned)((c->NP / 4 + 255) / 256), ATJUP_S_COUNT), 256, 0, c->stream>>>(s);
         c->launches++;
         break;
+    }
     case MICRO_DIAG:
         diagnostics_kernel<<<gcell, TB, 0, c->stream>>>(diag_args(c));
         c->launches++;

@@ -117,18 +117,14 @@ void free_all(AtjupCtx* c) {
     for (int q = 0; q < 4; q++) {
         cudaFree(c->X1[q]); cudaFree(c->X2[q]); cudaFree(c->acc[q]);
     }
-    for (auto& p : c->kr) { cudaFree(p); p = nullptr; }
-    for (auto& p : c->kf) { cudaFree(p); p = nullptr; }
     cudaFree(c->src); cudaFree(c->tmp); cudaFree(c->tmp2); cudaFree(c->red); cudaFree(c->stage);
     cudaFree(c->buoy_ref); cudaFree(c->zm); cudaFree(c->dvc); cudaFree(c->dvrow);
     cudaFree(c->mca_bounds); cudaFree(c->mca_flags); cudaFree(c->mca_slots); cudaFree(c->mca_stats);
     cudaFree(c->mca_pairs);
-    cudaFree(c->solve_b); cudaFree(c->dsum); cudaFree(c->counters);
-    if (c->hsum) cudaFreeHost(c->hsum);
+    cudaFree(c->solve_b); cudaFree(c->counters);
     cudaFree(c->solid); cudaFree(c->nbflags); cudaFree(c->topo); cudaFree(c->floor_hi); cudaFree(c->run); cudaFree(c->geo); cudaFree(c->cor_col);
     cudaFree(c->sin_the); cudaFree(c->rad); cudaFree(c->cell_vbar0); cudaFree(c->cell_ubar0);
-    cudaFree(c->solid_list); cudaFree(c->amb_rows); cudaFree(c->yw);
-    cudaFree(c->line_a); cudaFree(c->line_c); cudaFree(c->line_m);
+    cudaFree(c->solid_list); cudaFree(c->amb_rows);
     for (auto e : c->tev) cudaEventDestroy(e);
     c->tev.clear();
 }

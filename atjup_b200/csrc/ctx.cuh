@@ -107,12 +107,7 @@ struct AtjupCtx {
     double* zm = nullptr;        // [4 * jm] zonal means for the top sponge
     double* dvc = nullptr;       // [jm * KP] column means of v
     double* dvrow = nullptr;     // [jm]
-    // Krylov solver vectors (allocated on first RESIDUAL solve)
-    double* kr[8] = {};
-    float* kf[8] = {};
     double* solve_b = nullptr;   // external right-hand side
-    double* dsum = nullptr;      // [ATJUP_MAX_SOLVE_PARTIALS * 4] dot-product partials
-    double* hsum = nullptr;      // pinned host copy of the final dot products
     unsigned long long* counters = nullptr;  // [8] event counters of the last satadj call
     double* lin = nullptr;       // scratch of the RK4 tangent-linear / adjoint (adjoint.cu)
     double* itlin = nullptr;     // scratch of the iteration's tangent-linear / adjoint (iteration_lin.cu)
@@ -133,10 +128,6 @@ struct AtjupCtx {
     int n_solid = 0;
     int32_t* amb_rows = nullptr;   // (i, j) rows that contain solid cells
     int n_amb_rows = 0;
-    double* yw = nullptr;          // [NP] left null vector weight a_i d_j on fluid unknowns
-    double* line_a = nullptr;      // radial line factors for the preconditioner
-    double* line_c = nullptr;
-    double* line_m = nullptr;
     double yw_sum = 0.0;
     void* solver = nullptr;           // residual-solver state (solver.cu), built on first use
     void* cone = nullptr;             // projection around the obstacle (cone.cu), built on first use

@@ -8,12 +8,12 @@
 // species floor at 0, the NaN-safe clamp of k* into [0, k_max], omega* >= 1e-10).
 //
 // A scalar's right-hand side needs its own 7-point stencil, the cell's velocities and nue, and
-// its frozen sources, and no other scalar. So the species kernel is one thread per cell and
-// species (k fastest, coalesced): it reads the stage input at the cell and its six neighbours (the
+// its frozen sources, and no other scalar. So the species kernel is one thread per cell, the species
+// in turn (k fastest, coalesced): it reads the stage input at the cell and its six neighbours (the
 // k neighbours from the warp's own loads, the i and j neighbours mostly from L2), the
-// time-level-n value and the accumulator, and writes the next stage input and the accumulator --
-// 6 to 8 doubles of DRAM traffic per species per cell per stage. The closure kernel adds the nine velocity gradients its production
-// term needs. Both kernels read the same stage input velocities as the dynamics kernel of the
+// time-level-n value and the frozen sources, and writes the next stage input -- 3 to 6 doubles of DRAM
+// traffic per species per cell per stage. The closure kernel adds the nine velocity gradients its
+// production term needs. Both kernels read the same stage input velocities as the dynamics kernel of the
 // stage, and write only scalar buffers, so they are ordered freely against it.
 //
 // Non-integrated cells (the radial walls, three rows next to each pole, the seam copy, solid

@@ -28,6 +28,7 @@
 // direction reads z, and its share of rho comes from the column sums. Every reduction ends in the
 // kernel that forms it.
 #include "ctx.cuh"
+#include "line_role.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -320,7 +321,6 @@ direction_kernel(double* __restrict__ d, double* __restrict__ p, const T* __rest
 // with one thread per column and the factors as 3-D fields; 29 us that way with row tables, which
 // leaves a 41x61x97 shell 177 warps of 39 levels in sequence: 20 us there, 12 us with segments).
 // The factors are read as m = 1 / pivot, al = -lower m, c = -upper m.
-constexpr int LSEG = 10, LWARPS = 8;
 template <typename T>
 struct LineMaps {
     T map[LWARPS][2][32];         // each segment's affine map, per column
@@ -335,9 +335,9 @@ __device__ __forceinline__ void line_segment(double (&rn)[LSEG], const double (&
                                              int len, int n, const T* __restrict__ fm,
                                              const T* __restrict__ fa, const T* __restrict__ fc,
                                              unsigned fs, bool act, bool init, double mean,
-                                             double alpha, double dj, int S, int s, int w,
+                                             double alpha, double dj, const LineRole& R, int w,
                                              LineMaps<T>& M, double* g, double (&v)[3]) {
-    const int lane = threadIdx.x & 31, w0 = w - s;
+    const int lane = threadIdx.x & 31, s = R.s, S = R.S, w0 = R.w0;
     T x[LSEG], A = 1, B = 0;
     double gs = 0.0, ends = 0.0, rr = 0.0;
     // (read-only loads for the columns' own factors: they may move above the stores to r and z)
@@ -356,7 +356,7 @@ __device__ __forceinline__ void line_segment(double (&rn)[LSEG], const double (&
         A *= al;
         B = al * B + x[u];
     }
-    if (h == 0) ends = rn[0];
+    if (h == 0 && len > 0) ends = rn[0];
 #pragma unroll
     for (int u = 0; u < LSEG; u++)
         if (h + u == n - 1 && u < len) ends += rn[u];
@@ -417,8 +417,9 @@ line_kernel(const double* b, double* r, const double* __restrict__ qv, T* z, Lin
     extern __shared__ __align__(16) unsigned char line_smem[];
     __shared__ LineMaps<T> M;
     const int n = q.im - 2, N = q.km - 1, J = q.jm - 2;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, s = w % S, cw = w / S, CW = LWARPS / S;
-    const int kb = (N + 32 * CW - 1) / (32 * CW), h = s * LSEG, len = min(LSEG, n - h);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, CW = LWARPS / S;
+    const LineRole R = line_role(w, S);
+    const int kb = (N + 32 * CW - 1) / (32 * CW), h = R.s * LSEG, len = R.on ? min(LSEG, n - h) : 0;
     T* sf = reinterpret_cast<T*>(line_smem);      // the row's factors: m, al, c
     const unsigned plane = (unsigned)q.jm * q.KP;                // every index is below 2^32
     double v[3] = {0.0, 0.0, 0.0};                // r.r, y.(r z), y.r
@@ -426,10 +427,10 @@ line_kernel(const double* b, double* r, const double* __restrict__ qv, T* z, Lin
     pdl_wait();
     const double alpha = INIT ? 0.0 : scal[SC_ALPHA], mean = INIT ? 0.0 : scal[SC_MEAN];
     for (int t = blockIdx.x; t < kb * J; t += gridDim.x) {
-        // LWARPS need not be a multiple of S, nor N of the block's columns: the threads beyond
-        // work on the row's last column and store nothing
-        const int j = t / kb + 1, kk = ((t - (j - 1) * kb) * CW + cw) * 32 + lane;
-        const bool act = cw < CW && kk < N;
+        // N need not be a multiple of the block's columns: the lanes beyond work on the row's last column
+        // and store nothing. A warp without a group (S does not divide LWARPS) has no levels.
+        const int j = t / kb + 1, kk = ((t - (j - 1) * kb) * CW + R.group) * 32 + lane;
+        const bool act = R.on && kk < N;
         const int k = min(kk, N - 1);
         const unsigned o = plane + (unsigned)j * q.KP + k + (unsigned)h * plane;
         double rn[LSEG], qq[LSEG];
@@ -439,7 +440,7 @@ line_kernel(const double* b, double* r, const double* __restrict__ qv, T* z, Lin
                 rn[u] = INIT ? b[o + u * plane] : r[o + u * plane];
                 qq[u] = INIT ? 0.0 : qv[o + u * plane];
             }
-        const int sl = slot[(size_t)(j - 1) * N + k];
+        const int sl = R.on ? slot[(size_t)(j - 1) * N + k] : -1;
         __syncthreads();                          // the last tile's factors and maps are read
         for (int i = threadIdx.x; i < 3 * n; i += blockDim.x) {
             const int f = i / n;
@@ -451,7 +452,7 @@ line_kernel(const double* b, double* r, const double* __restrict__ qv, T* z, Lin
         double* gc = g + (size_t)(j - 1) * N + k;
         if (!irregular) {
             line_segment<T, true>(rn, qq, r, z, o, plane, h, len, n, sf + h, sf + n + h, sf + 2 * n + h,
-                                  1, act, INIT, mean, alpha, dj, S, s, w, M, gc, v);
+                                  1, act, INIT, mean, alpha, dj, R, w, M, gc, v);
         } else {
             const size_t ro = (size_t)(j - 1) * n + h;
             const T *m = L.rm + ro, *al = L.ra + ro, *c = L.rc + ro;
@@ -462,7 +463,7 @@ line_kernel(const double* b, double* r, const double* __restrict__ qv, T* z, Lin
                 fs = n_irr;
             }
             line_segment<T, false>(rn, qq, r, z, o, plane, h, len, n, m, al, c, fs, act, INIT, mean,
-                                   alpha, dj, S, s, w, M, gc, v);
+                                   alpha, dj, R, w, M, gc, v);
         }
     }
     if (grid_sum(v, part, ticket)) {

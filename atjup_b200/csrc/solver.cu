@@ -989,10 +989,14 @@ void free_lines(Lines<T>& l) {
     l = Lines<T>();
 }
 
-// Shared memory of the DFT kernels (tables and folds), 0 when the ring is too long for it
+// Dynamic shared memory of the DFT kernels (tables and folds), 0 when the ring is too long for it. With the
+// kernels' own (17 KB in the inverse) it exceeds a launch's default 48 KB from 954 meridians on, so both
+// are allowed DFT_SMEM whatever the ring: a limit set to one ring's need would also be the one left for
+// another context with a longer ring.
+constexpr size_t DFT_SMEM = 200 * 1024;
 size_t dft_bytes(int N) {
     const size_t b = sizeof(double2) * (size_t)(N + N / 8 + 1) + sizeof(double) * DFT_ROWS * ((size_t)N + 4);
-    return b <= 200 * 1024 ? b : 0;
+    return b <= DFT_SMEM ? b : 0;
 }
 
 // Build y, the cell codes, the line factors and the coarse (column-mode) factors from the mask and
@@ -1129,10 +1133,8 @@ int setup(AtjupCtx* c, Solver* S) {
         (rc_ = alloc_zero(&S->scal, SC_COUNT)) || (rc_ = alloc_zero(&S->yw, NP)) ||
         (rc_ = alloc_zero(&S->code, NP)))
         return rc_;
-    if (dft_bytes(N) > 48 * 1024) {
-        ATJUP_CUDA(cudaFuncSetAttribute(dft_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dft_bytes(N)));
-        ATJUP_CUDA(cudaFuncSetAttribute(dft_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dft_bytes(N)));
-    }
+    ATJUP_CUDA(cudaFuncSetAttribute(dft_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DFT_SMEM));
+    ATJUP_CUDA(cudaFuncSetAttribute(dft_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DFT_SMEM));
     if (!dft_bytes(N) && (rc_ = alloc_zero(&S->fold, (size_t)(J + 1) * (N + 4)))) return rc_;
     if ((rc_ = upload_as(&S->l64.ra, ra)) || (rc_ = upload_as(&S->l64.rc, rc)) ||
         (rc_ = upload_as(&S->l64.rm, rm)) || (rc_ = upload_as(&S->l64.ia, ia)) ||

@@ -15,7 +15,10 @@ static thread_local std::string g_err;
 
 void set_error(const std::string& msg) { g_err = msg; }
 
+// The error is reported here, so it is taken off the runtime too: left there, the next launch check of any
+// model (or of torch) in the process would report it as its own.
 int cuda_status(cudaError_t e, const char* what) {
+    cudaGetLastError();
     g_err = std::string(what) + ": " + cudaGetErrorString(e);
     return ATJUP_ERR_CUDA;
 }

@@ -64,6 +64,7 @@ constexpr int SNAP_EVERY = 64;           // wavefront steps between snapshots
 constexpr int CONE_CLUSTER = 4;          // blocks per level (fewer when the GPU cannot hold them)
 constexpr size_t CONE_SMEM_CAP = 200 * 1024;
 constexpr int CHECK_STEPS = 16;          // wavefront steps between stopping tests
+constexpr int DRAIN_POLLS = 1 << 20;     // of the rows still under way when a solve is given up
 // per box row: aN, aS, aL, A of a plain cell, 1 / A, s, s dphi (and one unused: rows of 64 bytes, read
 // two doubles at a time)
 constexpr int NROW = 8;
@@ -128,8 +129,17 @@ struct ConeArgs {
     double* w;
     const uint8_t* solid;
     const double* rad;
-    int jm, km, KP, H, C, ring_max;
+    int jm, km, KP, H, C, ring_max, polls;
     double dr, dthe, dphi;
+};
+
+// RowForm: a block's barriers for the rows of its neighbours, [2 side + colour], north's side first; and what
+// is kept once a wait on one of them has given up.
+struct RowWaits {
+    unsigned long long bar[4];
+    int owed[4];                // rows that came after it, which no wait has taken
+    int gave[2];                // the colour whose wait gave up, per side
+    int lost;                   // any warp of the block gave up
 };
 
 // A block's band of a level's box as the kernel sees it. Local row la = 1..nb is box row
@@ -144,8 +154,9 @@ struct Box {
     const double* rows;         // [NJ][NROW], indexed by box row
     unsigned long long* ring;   // [2 R]: largest change, largest |phi| of sweep t at t mod R
     double *push_n, *push_s;    // the neighbours' copies of this band's first and last row (colour 0), or null
-    unsigned bar_n, bar_s;      // RowForm: those copies' barriers there, and this block's own (shared addresses)
-    unsigned bar;
+    unsigned bar_n, bar_s;      // RowForm: those copies' barriers there (shared addresses)
+    RowWaits* waits;            // and this block's own
+    int polls;                  // of a wait for a neighbour's row
     int NJ, NK, PW, D, R;       // R a power of two
     int nb, A0;
     bool div;
@@ -241,8 +252,10 @@ struct WordForm {
         la_step = (THREADS / 32) >> lg;
     }
     __device__ __forceinline__ void load(const Box&) {}
-    __device__ __forceinline__ bool settle(const Box&) { return true; }
+    __device__ __forceinline__ void settle(const Box&) {}
+    __device__ __forceinline__ void drain(const Box&) {}
     __device__ __forceinline__ void end_step() { cluster_sync(); }
+    static constexpr bool WAITS = false;
     __device__ static bool odd_row(const Box&) { return false; }
     template <bool PAR, int c, bool REDUCE>
     __device__ __forceinline__ void step(const Box& B, int tau, unsigned t2) {
@@ -293,7 +306,12 @@ struct WordForm {
 // colour, and waits for the neighbour's row before its own next step (two barriers a side: a row of
 // one colour is sent only after the neighbour's row of the other colour arrived, so a phase is over before the
 // next one's bytes come). A cluster barrier for each step took 725 cycles, more than the step's work.
+//
+// A wait gives up after B.polls polls (the blocks of a cluster run together, so a row is at most a few polls
+// away). The warp then goes on without waiting, so that no other waits for it, until the stopping test, where
+// every block of the cluster learns of it and the level's solve ends.
 struct RowForm {
+    static constexpr bool WAITS = true;
     static constexpr int ROWS = 28, THREADS = 32 * ROWS, WORDS = 64;
     double val[2][2];                    // [phase][word]
     double md[2], mp[2];                 // largest change and |phi| of the sweep in each word
@@ -337,7 +355,7 @@ struct RowForm {
         if (edge) {
             push = (unsigned)__cvta_generic_to_shared(to) + 8 * m;
             bar_there = la == 1 ? B.bar_n : B.bar_s;
-            bar_here = B.bar + (la == 1 ? 0 : 16);
+            bar_here = (unsigned)__cvta_generic_to_shared(&B.waits->bar[2 * side()]);
         }
         waiting = -1;
         load(B);
@@ -350,20 +368,53 @@ struct RowForm {
             val[P][1] = x.y;
         }
     }
-    // waits for the neighbour's row of the last step; false (from then on) when it did not come
-    __device__ __forceinline__ bool settle(const Box& B) {
-        if (waiting < 0) return !dead;
-        const unsigned b = bar_here + 8 * waiting, ph = (phases >> waiting) & 1;
-        if (lane == 0)
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(b), "r"(8 * WORDS) : "memory");
-        unsigned done = dead;
-        for (int tries = 0; !done && tries < (1 << 16); tries++)
+    __device__ __forceinline__ int side() const { return la == 1 ? 0 : 1; }
+    __device__ static bool poll(unsigned bar, unsigned parity, int polls) {
+        unsigned done = 0;
+        for (int tries = 0; !done && tries < polls; tries++)
             asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-                         " selp.u32 %0, 1, 0, p;\n}" : "=r"(done) : "r"(b), "r"(ph) : "memory");
-        if (!done) dead = true;
-        phases ^= 1u << waiting;
+                         " selp.u32 %0, 1, 0, p;\n}" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        return done;
+    }
+    __device__ __forceinline__ void expect(unsigned bar, int rows) {
+        if (lane == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(8 * WORDS * rows) : "memory");
+    }
+    // waits for the neighbour's row of the last step, until a wait has given up
+    __device__ __forceinline__ void settle(const Box& B) {
+        if (waiting < 0) return;
+        if (dead) {
+            if (lane == 0) B.waits->owed[2 * side() + waiting]++;
+        } else {
+            expect(bar_here + 8 * waiting, 1);
+            const bool came = poll(bar_here + 8 * waiting, (phases >> waiting) & 1, B.polls);
+            dead = __any_sync(0xffffffffu, !came);
+            if (!dead) phases ^= 1u << waiting;
+            else if (lane == 0) {
+                B.waits->gave[side()] = waiting;
+                B.waits->lost = 1;
+            }
+        }
         waiting = -1;
-        return !dead;
+    }
+    // After a wait has given up and every block has taken its last step: takes the rows that are still
+    // under way, which may land in this block's memory until then.
+    __device__ __forceinline__ void drain(const Box& B) {
+        if (!edge || !dead) return;
+#pragma unroll 1
+        for (int c = 0; c < 2; c++) {
+            const unsigned b = bar_here + 8 * c;
+            unsigned ph = (phases >> c) & 1;
+            if (B.waits->gave[side()] == c) {
+                poll(b, ph, DRAIN_POLLS);
+                ph ^= 1;
+            }
+            const int rows = B.waits->owed[2 * side() + c];
+            if (rows > 0) {
+                expect(b, rows);
+                poll(b, ph, DRAIN_POLLS);
+            }
+        }
     }
     template <int P, int c, bool REDUCE>
     __device__ __forceinline__ void phase(const Box& B, int tau, unsigned t2) {
@@ -461,8 +512,17 @@ __device__ void band_copy(double* phi, int cs, double* packed, int nb, int PW, b
         }
 }
 
+// a wait of some block of the cluster has given up (after a cluster barrier)
+__device__ __forceinline__ bool cluster_lost(const Box& B, int C) {
+    cg::cluster_group cl = cg::this_cluster();
+    int any = 0;
+    for (int r = 0; r < C; r++) any |= *cl.map_shared_rank(&B.waits->lost, r);
+    return any;
+}
+
 // Lexicographic SOR of one level's solve as the pipelined wavefront on the cluster; returns the
-// reference's sweep count `it` (the converged sweep, or CONE_MAXIT + 1 without convergence).
+// reference's sweep count `it` (the converged sweep, or CONE_MAXIT + 1 without convergence), or -1 in every
+// block when a neighbour's row did not come.
 // snap: this block's snapshot ring, n_snap slots of 2 (nbmax + 2) PW doubles.
 template <class Form, bool PAR>
 __device__ __forceinline__ int cone_sor(const Box& B, Form& T, double* snap, int slot_sz, int n_snap, int* snap_tag, int* t_found, int C) {
@@ -502,11 +562,14 @@ __device__ __forceinline__ int cone_sor(const Box& B, Form& T, double* snap, int
                     pmax = fmax(pmax, __shfl_xor_sync(0xffffffffu, pmax, o));
                 }
                 const unsigned conv = __ballot_sync(0xffffffffu, t <= t_done && dmax <= CONE_TOL * fmax(pmax, 1.0e-30));
-                if (lane == 0) *t_found = conv ? t_next + ((__ffs(conv) - 1) >> 2) : 0;
+                bool lost = false;
+                if constexpr (Form::WAITS)
+                    lost = __any_sync(0xffffffffu, lane < C && *cl.map_shared_rank(&B.waits->lost, lane < C ? lane : 0));
+                if (lane == 0) *t_found = lost ? -1 : conv ? t_next + ((__ffs(conv) - 1) >> 2) : 0;
             }
             block_sync();
             t_conv = *t_found;
-            if (t_conv > 0) break;
+            if (t_conv != 0) break;
             t_next = t_done + 1;
             if (t_done == CONE_MAXIT) break;
         }
@@ -542,6 +605,10 @@ __device__ __forceinline__ int cone_sor(const Box& B, Form& T, double* snap, int
         T.settle(B);
         block_sync();
     }
+    if constexpr (Form::WAITS) {
+        cluster_sync();          // the blocks' last waits are over
+        if (cluster_lost(B, C)) it = -1;
+    }
     return it;
 }
 
@@ -565,19 +632,25 @@ __global__ void __launch_bounds__(Form::THREADS, 1) cone_kernel(ConeArgs A) {
     double* phi_local = reinterpret_cast<double*>(B.ring + 2 * A.ring_max);
     double *rows, *tab;
     B.push_n = B.push_s = nullptr;
-    __shared__ __align__(8) unsigned long long bars[4];        // north's two colours, south's two
+    __shared__ RowWaits waits;
     Form T;
-    if constexpr (std::is_same<Form, RowForm>::value) {
-        B.bar = (unsigned)__cvta_generic_to_shared(bars);
+    if constexpr (Form::WAITS) {
+        B.waits = &waits;
+        B.polls = A.polls;
         T.phases = 0;
         T.dead = false;
         if (threadIdx.x == 0) {
-            for (int x = 0; x < 4; x++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(B.bar + 8 * x) : "memory");
+            for (int x = 0; x < 4; x++) {
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"((unsigned)__cvta_generic_to_shared(&waits.bar[x])) : "memory");
+                waits.owed[x] = 0;
+            }
+            waits.gave[0] = waits.gave[1] = -1;
+            waits.lost = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         // a row stored in the neighbour to the north is that block's southern one
-        if (r > 0) B.bar_n = (unsigned)__cvta_generic_to_shared(cl.map_shared_rank(bars + 2, r - 1));
-        if (r < C - 1) B.bar_s = (unsigned)__cvta_generic_to_shared(cl.map_shared_rank(bars, r + 1));
+        if (r > 0) B.bar_n = (unsigned)__cvta_generic_to_shared(cl.map_shared_rank(waits.bar + 2, r - 1));
+        if (r < C - 1) B.bar_s = (unsigned)__cvta_generic_to_shared(cl.map_shared_rank(waits.bar, r + 1));
     }
     if constexpr (SMEM) {
         B.cs = (nbmax + 2) * PW;
@@ -673,6 +746,23 @@ __global__ void __launch_bounds__(Form::THREADS, 1) cone_kernel(ConeArgs A) {
         const int it = Form::odd_row(B) ? cone_sor<Form, true>(B, T, snap, slot_sz, L.n_snap, snap_tag, &t_found, C)
                                         : cone_sor<Form, false>(B, T, snap, slot_sz, L.n_snap, snap_tag, &t_found, C);
         __syncthreads();
+        if (Form::WAITS && it < 0) {
+            // The level has no result: its winds are NaN, as the Runge-Kutta stage marks cells whose inputs did
+            // not come, and the warm start stays the last call's.
+            T.drain(B);
+            const double nan = __longlong_as_double(0x7ff8000000000000ll);
+            for (int x = threadIdx.x; x < nb * NK; x += blockDim.x) {
+                const int la = 1 + x / NK, a = A0 + la - 1, bp = x % NK + 1;
+                const int cc = (a + 1 + bp) & 1;
+                if (B.info[cc * B.ics + (la - 1) * PW + (bp >> 1)] & CF_SOLID) continue;
+                const size_t cix = ((size_t)i * A.jm + (L.jlo + a)) * A.KP + (L.klo + bp - 1);
+                A.v[cix] = A.w[cix] = nan;
+            }
+            if (r == 0 && threadIdx.x == 0)
+                for (int q = pass; q < 2; q++) A.stats[2 * lvl + q] = -1;
+            cl.sync();           // the flags of every block are read
+            return;
+        }
         // v and w of the band incremented by the average of the two face corrections
         // (InitValues_Jup.cpp:1785-1793), a wall face's correction being minus the cell's velocity
         for (int x = threadIdx.x; x < nb * NK; x += blockDim.x) {
@@ -697,10 +787,8 @@ __global__ void __launch_bounds__(Form::THREADS, 1) cone_kernel(ConeArgs A) {
                 prev[(size_t)col * (NJ + 2) * PW + (size_t)(A0 + 1) * PW + rr] = phi_local[col * B.cs + PW + rr];
             }
         if (r == 0 && threadIdx.x == 0) A.stats[2 * lvl + pass] = it;
-        const bool lost = __syncthreads_or(!T.settle(B)) != 0;      // a neighbour's row never came
         // every block is past its last store to a neighbour, and the warm start is read after it is whole
         cl.sync();
-        if (lost && threadIdx.x == 0) A.stats[2 * lvl + pass] = -1;
     }
 }
 
@@ -957,6 +1045,7 @@ int launch_cone_projection(AtjupCtx* c) {
         A.jm = P.jm; A.km = P.km; A.KP = c->KP; A.H = cs->H;
         A.C = cs->C;
         A.ring_max = cs->ring_max;
+        A.polls = c->cone_polls;
         A.dr = P.dr; A.dthe = P.dthe; A.dphi = P.dphi;
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute at[1];
@@ -1007,6 +1096,18 @@ int atjup_gpu_cone_stats(AtjupCtx* c, int32_t* level_i, int32_t* sweeps, int32_t
         if (level_i) level_i[l] = cs->lv[l].i;
         if (sweeps) { sweeps[2 * l] = st[2 * l]; sweeps[2 * l + 1] = st[2 * l + 1]; }
     }
+    for (int l = 0; l < nl; l++)
+        if (st[2 * l] < 0 || st[2 * l + 1] < 0) {
+            set_error("cone projection: a wait for a neighbour's row gave up on level " +
+                      std::to_string(cs->lv[l].i) + "; its winds are NaN");
+            return ATJUP_ERR_NONFINITE;
+        }
+    return ATJUP_OK;
+}
+
+int atjup_gpu_cone_wait_limit(AtjupCtx* c, int32_t polls) {
+    if (!c || polls < 0) { set_error("cone_wait_limit: bad argument"); return ATJUP_ERR_ARG; }
+    c->cone_polls = polls;
     return ATJUP_OK;
 }
 

@@ -131,6 +131,7 @@ struct AtjupCtx {
     double yw_sum = 0.0;
     void* solver = nullptr;           // residual-solver state (solver.cu), built on first use
     void* cone = nullptr;             // projection around the obstacle (cone.cu), built on first use
+    int cone_polls = 1 << 16;         // of its waits for a neighbour block's row
 
     // instrumentation: kernel launches issued, and CUDA-event timing per kernel class
     long long launches = 0;

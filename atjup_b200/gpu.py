@@ -64,6 +64,7 @@ def load_library() -> ctypes.CDLL:
     L.atjup_gpu_mixture_density.argtypes = [vp]
     L.atjup_gpu_balance_column_v.argtypes = [vp, ctypes.POINTER(dbl)]
     L.atjup_gpu_cone_project.argtypes = [vp]
+    L.atjup_gpu_cone_wait_limit.argtypes = [vp, i32]
     L.atjup_gpu_cone_stats.argtypes = [vp, ctypes.POINTER(i32), ctypes.POINTER(i32), i32,
                                        ctypes.POINTER(i32)]
     L.atjup_gpu_step.argtypes = [vp, i32, i32, ctypes.POINTER(_p.AtjupSolveOpts)]
@@ -468,7 +469,8 @@ class GpuModel:
 
     def cone_stats(self):
         """(levels i, sweeps [levels, 2]) of the last projection: SOR sweeps of the divergence
-        solve (0 when off) and of the wall-flux solve per level."""
+        solve (0 when off) and of the wall-flux solve per level. Raises when a level's solve was given
+        up (its winds are NaN)."""
         n = ctypes.c_int32()
         _check(self.L.atjup_gpu_cone_stats(self.ctx, None, None, 0, ctypes.byref(n)))
         lv = (ctypes.c_int32 * max(n.value, 1))()
@@ -476,6 +478,10 @@ class GpuModel:
         _check(self.L.atjup_gpu_cone_stats(self.ctx, lv, sw, n.value, ctypes.byref(n)))
         return (np.array(lv[:n.value], dtype=np.int32),
                 np.array(sw[:2 * n.value], dtype=np.int32).reshape(n.value, 2))
+
+    def cone_wait_limit(self, polls: int) -> None:
+        """atjup_gpu_cone_wait_limit: polls of the projection's waits between blocks of a level"""
+        _check(self.L.atjup_gpu_cone_wait_limit(self.ctx, int(polls)))
 
     def satadj(self, gas: str, gp: _p.AtjupGasParams, stats: bool = True):
         """SaturationAdjustmentJup(*this).run(gas, ...) (SaturationAdjustment.h:255-746) on the

@@ -266,9 +266,15 @@ int atjup_gpu_balance_column_v(AtjupCtx* ctx, double* vshift);
 int atjup_gpu_cone_project(AtjupCtx* ctx);
 /* The levels of the projection and the SOR sweeps of its last call, per level: sweeps[2 l] of the
  * divergence solve (0 when off), sweeps[2 l + 1] of the wall-flux solve (40001: not converged
- * within 40000 sweeps, the reference's count). Fills up to cap levels; *n_levels = all levels. */
+ * within 40000 sweeps, the reference's count). Fills up to cap levels; *n_levels = all levels.
+ * A level is shared by the blocks of a cluster, which wait for each other's edge rows for a limited
+ * number of polls. Should a wait give up, the level has no result: v and w of its box are NaN, its
+ * solves (from the one that gave up on) read -1 here, and this call, when cap > 0, returns
+ * ATJUP_ERR_NONFINITE with the arrays filled. */
 int atjup_gpu_cone_stats(AtjupCtx* ctx, int32_t* level_i, int32_t* sweeps, int32_t cap,
                          int32_t* n_levels);
+/* That limit, in polls (65536 by default; 0: every such wait gives up, which is how a test reaches it). */
+int atjup_gpu_cone_wait_limit(AtjupCtx* ctx, int32_t polls);
 
 /* The column balance of v for callers that cannot allocate device memory. No counterpart in the
  * reference: it computes what atjup_gpu_balance_column_v computes, on the caller's own device

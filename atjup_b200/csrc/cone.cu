@@ -43,11 +43,11 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
-#include <type_traits>
 #include <vector>
 
 #include <cooperative_groups.h>
 
+#include "cone_plan.cuh"
 #include "ctx.cuh"
 #include "quot.cuh"
 
@@ -61,13 +61,11 @@ constexpr double CONE_OMEGA = 1.9;       // InitValues_Jup.cpp:1726
 constexpr int CONE_MAXIT = 40000;        // InitValues_Jup.cpp:1728
 constexpr double CONE_TOL = 1.0e-10;     // InitValues_Jup.cpp:1761
 constexpr int SNAP_EVERY = 64;           // wavefront steps between snapshots
-constexpr int CONE_CLUSTER = 4;          // blocks per level (fewer when the GPU cannot hold them)
-constexpr size_t CONE_SMEM_CAP = 200 * 1024;
 constexpr int CHECK_STEPS = 16;          // wavefront steps between stopping tests
 constexpr int DRAIN_POLLS = 1 << 20;     // of the rows still under way when a solve is given up
 // per box row: aN, aS, aL, A of a plain cell, 1 / A, s, s dphi (and one unused: rows of 64 bytes, read
 // two doubles at a time)
-constexpr int NROW = 8;
+constexpr int NROW = CONE_NROW;
 enum { RC_N, RC_S, RC_L, RC_A, RC_RA, RC_SJ, RC_SD };
 
 // cell flags of the box (uint32 per cell: these bits, the special-cell index above bit 6)
@@ -102,13 +100,9 @@ struct ConeState {
     double* s = nullptr;                    // [jm] max(sinthe_min, |sin(the_j)|)
     int* stats = nullptr;                   // [2 * levels] sweeps of the last call
     int H = 0, M = 0;
-    int C = 1;                              // blocks (one cluster) per level
+    ConePlan plan{};
     int ring_max = 1;                       // the largest ring of the levels
-    bool smem_mode = true;
-    const void* kernel = nullptr;           // the form of cone_kernel for the levels' bands, and its threads
-    int threads = 0;
-    size_t smem = 0;                        // dynamic shared memory per block
-    int64_t n_phi = 0;
+    const void* kernel = nullptr;           // the plan's form of cone_kernel
 };
 
 namespace {
@@ -312,7 +306,7 @@ struct WordForm {
 // every block of the cluster learns of it and the level's solve ends.
 struct RowForm {
     static constexpr bool WAITS = true;
-    static constexpr int ROWS = 28, THREADS = 32 * ROWS, WORDS = 64;
+    static constexpr int ROWS = CONE_ROWS, THREADS = 32 * ROWS, WORDS = CONE_WORDS;
     double val[2][2];                    // [phase][word]
     double md[2], mp[2];                 // largest change and |phi| of the sweep in each word
     RowCoef R;
@@ -875,9 +869,9 @@ int cone_prepare(AtjupCtx* c) {
     auto* cs = new ConeState();
     cs->H = H;
     cs->M = M;
-    std::vector<uint32_t> info;
-    std::vector<int32_t> spec;
-    int64_t n_phi = 0, n_snap = 0, n_tab = 0, n_row = 0;
+    // the boxes, and the flags of their cells row by row
+    std::vector<std::vector<uint32_t>> flags;
+    std::vector<ConeBox> boxes;
     for (int i = 1; i < im - 1; i++) {
         int jmin = jm, jmax = -1, kmin = km, kmax = -1;
         for (int j = 0; j < jm; j++)
@@ -893,8 +887,7 @@ int cone_prepare(AtjupCtx* c) {
         ConeLevel L{};
         L.i = i; L.jlo = jlo; L.klo = klo;
         L.NJ = jhi - jlo + 1; L.NK = khi - klo + 1;
-        // words per row and colour, halo included; RowForm's lanes have all their words in every row
-        L.PW = std::max((L.NK + 3) / 2, RowForm::WORDS);
+        L.PW = (L.NK + 3) / 2;                       // words per row and colour, halo included
         L.D = L.NJ + L.NK - 2;
         L.ring = 1;
         // a power of two above the sweeps in flight and those that wait for their stopping test
@@ -905,13 +898,10 @@ int cone_prepare(AtjupCtx* c) {
             set_error("cone projection: box too large");
             return ATJUP_ERR_UNSUPPORTED;
         }
-        L.info_off = (int64_t)info.size();
-        L.spec_off = (int64_t)spec.size();
-        info.resize(info.size() + 2 * (size_t)L.NJ * L.PW, CF_SOLID);   // unused words: skipped
+        std::vector<uint32_t> fl((size_t)L.NJ * L.NK);
         for (int a = 0; a < L.NJ; a++)
             for (int b = 0; b < L.NK; b++) {
                 const int j = jlo + a, k = klo + b;
-                const int e = (((a + b) & 1) * L.NJ + a) * L.PW + ((b + 1) >> 1);
                 uint32_t f = 0;
                 if (S(i, j, k)) f = CF_SOLID;
                 else {
@@ -924,87 +914,66 @@ int cone_prepare(AtjupCtx* c) {
                         const int entry = f & CF_WALL ? TAB_WALL : TAB_NEAR;
                         f |= (uint32_t)(L.n_tab / 2) << 6;
                         L.n_tab += entry;
-                        spec.push_back(e);
+                        L.n_spec++;
                     }
                 }
-                info[L.info_off + e] = f;
+                fl[(size_t)a * L.NK + b] = f;
             }
-        L.n_spec = (int)(spec.size() - L.spec_off);
-        const int64_t nphi = 2 * (int64_t)(L.NJ + 2) * L.PW;
-        L.phi_off = n_phi;  n_phi += nphi;
-        L.tab_off = n_tab;  n_tab += L.n_tab;
-        L.row_off = n_row;  n_row += NROW * (int64_t)L.NJ;
+        flags.push_back(std::move(fl));
+        boxes.push_back(ConeBox{L.NJ, L.NK, L.ring, L.n_tab});
         cs->ring_max = std::max(cs->ring_max, L.ring);
         cs->lv.push_back(L);
     }
     c->cone = cs;
-    cs->n_phi = n_phi;
     const size_t nl = cs->lv.size();
-    // blocks per level: a cluster of up to CONE_CLUSTER, each block a band of at least one row,
-    // the bands in shared memory; a level whose box does not fit runs as one block in HBM
-    int C = CONE_CLUSTER;
-    for (const ConeLevel& L : cs->lv) C = std::min(C, L.NJ);
-    auto smem_for = [&](int Cn) {
-        size_t mx = 0;
-        for (const ConeLevel& L : cs->lv) {
-            const size_t nbmax = (size_t)(L.NJ + Cn - 1) / Cn;
-            mx = std::max(mx, sizeof(double) * (2 * (nbmax + 2) * L.PW + NROW * (size_t)L.NJ +
-                                                (size_t)L.n_tab) +
-                                  sizeof(uint32_t) * 2 * nbmax * L.PW);
-        }
-        return mx + sizeof(unsigned long long) * 2 * (size_t)cs->ring_max;
+    auto kernel_of = [](const ConePlan& p) {
+        return p.row ? reinterpret_cast<const void*>(&cone_kernel<true, RowForm>)
+                     : p.smem ? reinterpret_cast<const void*>(&cone_kernel<true, WordForm>)
+                              : reinterpret_cast<const void*>(&cone_kernel<false, WordForm>);
     };
-    // the kernel for C blocks a level and its threads: a warp per row where every band allows it
-    auto form_for = [&](int Cn, int& threads) {
-        int rows = 1, words = 1, least = INT_MAX;
-        for (const ConeLevel& L : cs->lv) {
-            rows = std::max(rows, (L.NJ + Cn - 1) / Cn);
-            words = std::max(words, L.PW);
-            least = std::min(least, L.NJ / Cn);
-        }
-        const bool row = cs->smem_mode && least >= 2 && rows <= RowForm::ROWS && words <= RowForm::WORDS;
-        threads = row ? 32 * rows : WordForm::THREADS;
-        return row ? reinterpret_cast<const void*>(&cone_kernel<true, RowForm>)
-                   : cs->smem_mode ? reinterpret_cast<const void*>(&cone_kernel<true, WordForm>)
-                                   : reinterpret_cast<const void*>(&cone_kernel<false, WordForm>);
-    };
-    cs->smem_mode = nl > 0 && smem_for(std::max(C, 1)) <= CONE_SMEM_CAP;
-    if (!cs->smem_mode) C = 1;
-    C = std::max(C, 1);
-    // the largest cluster for which the GPU holds every level's cluster at once
-    for (; nl > 0 && C > 1; C--) {
-        const size_t sm = smem_for(C);
-        if (sm > CONE_SMEM_CAP) continue;
-        int threads = 0;
-        const void* form = form_for(C, threads);
-        if (cudaFuncSetAttribute(form, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) {
-            cudaGetLastError();
-            continue;
-        }
+    const ConePlan plan = cone_plan(boxes, [&](const ConePlan& p) {
+        int n_active = 0;
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3((unsigned)(nl * C));
-        cfg.blockDim = dim3(threads);
-        cfg.dynamicSmemBytes = sm;
+        at[0].val.clusterDim.x = p.C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3((unsigned)(nl * p.C));
+        cfg.blockDim = dim3(p.threads);
+        cfg.dynamicSmemBytes = p.bytes;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        int n_active = 0;
-        if (cudaOccupancyMaxActiveClusters(&n_active, form, &cfg) == cudaSuccess &&
-            n_active >= (int)nl)
-            break;
-        cudaGetLastError();
-    }
-    cs->smem = cs->smem_mode ? smem_for(C) : sizeof(unsigned long long) * 2 * (size_t)cs->ring_max;
-    cs->kernel = form_for(C, cs->threads);
+        const bool ok = cudaFuncSetAttribute(kernel_of(p), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.bytes) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&n_active, kernel_of(p), &cfg) == cudaSuccess && n_active >= (int)nl;
+        if (!ok) cudaGetLastError();
+        return ok;
+    });
+    cs->plan = plan;
+    cs->kernel = kernel_of(plan);
     if (nl > 0)
-        ATJUP_CUDA(cudaFuncSetAttribute(cs->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cs->smem));
-    cs->C = C;
-    for (ConeLevel& L : cs->lv) {
-        const int64_t nbmax = (L.NJ + C - 1) / C;
+        ATJUP_CUDA(cudaFuncSetAttribute(cs->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.bytes));
+    // the buffers' layout at the form's words per row
+    std::vector<uint32_t> info;
+    std::vector<int32_t> spec;
+    int64_t n_phi = 0, n_snap = 0, n_tab = 0, n_row = 0;
+    for (size_t l = 0; l < nl; l++) {
+        ConeLevel& L = cs->lv[l];
+        L.PW = cone_words(boxes[l], plan.row);
+        L.info_off = (int64_t)info.size();
+        L.spec_off = (int64_t)spec.size();
+        info.resize(info.size() + 2 * (size_t)L.NJ * L.PW, CF_SOLID);   // unused words: skipped
+        for (int a = 0; a < L.NJ; a++)
+            for (int b = 0; b < L.NK; b++) {
+                const uint32_t f = flags[l][(size_t)a * L.NK + b];
+                const int e = (((a + b) & 1) * L.NJ + a) * L.PW + ((b + 1) >> 1);
+                info[L.info_off + e] = f;
+                if (f & ~(uint32_t)CF_SOLID) spec.push_back(e);
+            }
+        L.phi_off = n_phi;  n_phi += 2 * (int64_t)(L.NJ + 2) * L.PW;
+        L.tab_off = n_tab;  n_tab += L.n_tab;
+        L.row_off = n_row;  n_row += NROW * (int64_t)L.NJ;
+        const int64_t nbmax = (L.NJ + plan.C - 1) / plan.C;
         L.snap_off = n_snap;
-        n_snap += (int64_t)C * L.n_snap * 2 * (nbmax + 2) * L.PW;
+        n_snap += (int64_t)plan.C * L.n_snap * 2 * (nbmax + 2) * L.PW;
     }
     ATJUP_CUDA(cudaMalloc(&cs->s, sizeof(double) * jm));
     ATJUP_CUDA(cudaMemcpy(cs->s, s.data(), sizeof(double) * jm, cudaMemcpyHostToDevice));
@@ -1023,7 +992,7 @@ int cone_prepare(AtjupCtx* c) {
         ATJUP_CUDA(cudaMemset(p, 0, sizeof(double) * n_phi));
     }
     ATJUP_CUDA(cudaMalloc(&cs->snap, sizeof(double) * n_snap));
-    if (!cs->smem_mode) {
+    if (!plan.smem) {
         ATJUP_CUDA(cudaMalloc(&cs->tab, sizeof(double) * std::max<int64_t>(n_tab, 1)));
         ATJUP_CUDA(cudaMalloc(&cs->rows, sizeof(double) * n_row));
     }
@@ -1043,17 +1012,17 @@ int launch_cone_projection(AtjupCtx* c) {
         A.u = c->f[ATJUP_F_U]; A.v = c->f[ATJUP_F_V]; A.w = c->f[ATJUP_F_W];
         A.solid = c->solid; A.rad = c->rad;
         A.jm = P.jm; A.km = P.km; A.KP = c->KP; A.H = cs->H;
-        A.C = cs->C;
+        A.C = cs->plan.C;
         A.ring_max = cs->ring_max;
         A.polls = c->cone_polls;
         A.dr = P.dr; A.dthe = P.dthe; A.dphi = P.dphi;
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = cs->C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3((unsigned)(cs->lv.size() * cs->C));
-        cfg.blockDim = dim3(cs->threads);
-        cfg.dynamicSmemBytes = cs->smem;
+        at[0].val.clusterDim.x = cs->plan.C; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3((unsigned)(cs->lv.size() * cs->plan.C));
+        cfg.blockDim = dim3(cs->plan.threads);
+        cfg.dynamicSmemBytes = cs->plan.bytes;
         cfg.stream = c->stream;
         cfg.attrs = at;
         cfg.numAttrs = 1;

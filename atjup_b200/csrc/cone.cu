@@ -931,6 +931,10 @@ int cone_prepare(AtjupCtx* c) {
                      : p.smem ? reinterpret_cast<const void*>(&cone_kernel<true, WordForm>)
                               : reinterpret_cast<const void*>(&cone_kernel<false, WordForm>);
     };
+    // the most any plan takes, not this one's need: the limit is the kernel's, and another context's plan may take more
+    auto allow = [&](const ConePlan& p) {
+        return cudaFuncSetAttribute(kernel_of(p), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CONE_SMEM_CAP);
+    };
     const ConePlan plan = cone_plan(boxes, [&](const ConePlan& p) {
         int n_active = 0;
         cudaLaunchConfig_t cfg{};
@@ -942,15 +946,14 @@ int cone_prepare(AtjupCtx* c) {
         cfg.dynamicSmemBytes = p.bytes;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        const bool ok = cudaFuncSetAttribute(kernel_of(p), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.bytes) == cudaSuccess &&
+        const bool ok = allow(p) == cudaSuccess &&
                         cudaOccupancyMaxActiveClusters(&n_active, kernel_of(p), &cfg) == cudaSuccess && n_active >= (int)nl;
         if (!ok) cudaGetLastError();
         return ok;
     });
     cs->plan = plan;
     cs->kernel = kernel_of(plan);
-    if (nl > 0)
-        ATJUP_CUDA(cudaFuncSetAttribute(cs->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.bytes));
+    ATJUP_CUDA(allow(plan));
     // the buffers' layout at the form's words per row
     std::vector<uint32_t> info;
     std::vector<int32_t> spec;

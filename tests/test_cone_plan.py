@@ -79,3 +79,23 @@ def test_every_plan_keeps_its_bounds(plans):
             if p["row"]:
                 assert x[0] // p["C"] >= 2 and -(-x[0] // p["C"]) <= 28 and p["threads"] >= 32 * -(-x[0] // p["C"])
     assert seen == {(1, 1), (0, 1), (0, 0)}
+
+
+def test_larger_constants_keep_a_box_in_shared_memory(plans):
+    """A box whose bands fit 200 KB with two doubles a special cell and six a row, up to 300 wall cells and 4000 near
+    ones, runs in clusters whatever the constants take now."""
+    rng = random.Random(7)
+    cases, sizes = [], []
+    while len(cases) < 300:
+        J, K = rng.randint(40, 400), rng.randint(40, 400)
+        wall, near = rng.randint(0, 300), rng.randint(0, 4000)
+        rows, words, ring = -(-J // 4), (K + 3) // 2, 1
+        while ring < (J + K - 2) // 2 + 2:
+            ring *= 2
+        small = 8 * (2 * (rows + 2) * words + 6 * J + 2 * (wall + near)) + 8 * rows * words + 16 * ring
+        if 150 * 1024 < small <= 200 * 1024:
+            cases.append((DEFAULT_SMS, [box(J, K, 8 * wall + 2 * near)]))
+            sizes.append(small)
+    assert max(sizes) > 195 * 1024
+    for p in plans(cases):
+        assert p["smem"] and p["C"] == 4

@@ -11,7 +11,8 @@ namespace atjup {
 constexpr int CONE_CLUSTER = 4;          // blocks per level (fewer when the GPU cannot hold them)
 // Dynamic shared memory of a block, of the 227 KB a block may have. The bands' constants (a wall cell's eight
 // doubles, a row's eight) take up to some 24 KB more than two doubles a special cell and six a row would: a box whose
-// bands fit 200 KB so must not leave shared memory for them (two levels of 299 x 179, a call from cold: 1150 ms on HBM, 246 so, 347 with the former kernel).
+// bands fit 200 KB so must not leave shared memory for them (two levels of 299 x 179, a call from cold: 1150 ms on
+// HBM, 246 so, 347 with the former kernel).
 constexpr size_t CONE_SMEM_CAP = 224 * 1024;
 constexpr int CONE_NROW = 8;             // doubles of constants per box row
 constexpr int CONE_ROWS = 28, CONE_WORDS = 64;   // the most rows of a band a warp per row takes, and its words

@@ -530,24 +530,23 @@ __global__ void fluxlim_kernel(MicroArgs a) {
     const double sinthe = dmax(a.mc.polar_divisor_floor, fabs(a.sin_the[j]));
     const double inv_rm = quot1(1.0, rm);
     const double inv_rmsinthe = quot1(1.0, rm * sinthe);
+    // n / (df + eps of its sign), by the magnitude: the quotients take positive divisors
+    auto over_eps = [&](double n, double df) { return quot1(df >= 0.0 ? n : -n, fabs(df) + eps); };
     double corr = 0.0;
     {
         const double df = q_rp - q, db = q - q_rm;
-        const double denom = df + (df >= 0.0 ? eps : -eps);
-        const double r = quot1((u >= 0.0) ? db : (i + 2 < a.im ? Q[c + 2 * plane] : q_rp) - q_rp, denom);
+        const double r = over_eps((u >= 0.0) ? db : (i + 2 < a.im ? Q[c + 2 * plane] : q_rp) - q_rp, df);
         corr += quot1((1.0 - superbee_phi(r)) * fabs(u) * (df - db), 2.0 * a.dr);
     }
     {
         const double df = q_tp - q, db = q - q_tm;
-        const double denom = df + (df >= 0.0 ? eps : -eps);
         const double q_far = (j + 2 < a.jm) ? Q[c + 2 * a.KP] : ((4.0 / 3.0) * q_tp - (1.0 / 3.0) * q);
-        const double r = quot1((v >= 0.0) ? db : q_far - q_tp, denom);
+        const double r = over_eps((v >= 0.0) ? db : q_far - q_tp, df);
         corr += quot1((1.0 - superbee_phi(r)) * fabs(v) * inv_rm * (df - db), 2.0 * a.dthe);
     }
     {
         const double df = q_pp - q, db = q - q_pm;
-        const double denom = df + (df >= 0.0 ? eps : -eps);
-        const double r = quot1((w >= 0.0) ? db : Q[row + wrap(k + 2)] - q_pp, denom);
+        const double r = over_eps((w >= 0.0) ? db : Q[row + wrap(k + 2)] - q_pp, df);
         corr += quot1((1.0 - superbee_phi(r)) * fabs(w) * inv_rmsinthe * (df - db), 2.0 * a.dphi);
     }
     a.fluxlim[c] = corr;

@@ -158,6 +158,8 @@ int timer_begin(AtjupCtx* c, int cls, cudaStream_t st);
 void timer_end(AtjupCtx* c, int slot, cudaStream_t st);
 int cuda_status(cudaError_t e, const char* what);
 
+constexpr int MAX_GRID_Z = 65535;     // blocks of a grid along y and z
+
 inline size_t cell(const AtjupCtx* c, int i, int j, int k) {
     return ((size_t)i * c->P.jm + j) * c->KP + k;
 }

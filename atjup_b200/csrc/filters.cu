@@ -286,6 +286,11 @@ int filter_tables(AtjupCtx* c, const int32_t* topo) {
 int launch_shapiro_n(AtjupCtx* c, double* const* f, int n, int order, double strength, int passes,
                      int use_topo) {
     const AtjupParams& P = c->P;
+    if ((long)P.im * n > MAX_GRID_Z) {         // a level and field per blockIdx.z: the fields one by one
+        for (int x = 0; x < n; x++)
+            if (int rc = launch_shapiro_n(c, f + x, 1, order, strength, passes, use_topo)) return rc;
+        return ATJUP_OK;
+    }
     FiltConst q{};
     q.im = P.im; q.jm = P.jm; q.km = P.km; q.KP = c->KP;
     q.use_topo = use_topo;

@@ -633,28 +633,31 @@ __global__ void vbal_row_T_kernel(const double* __restrict__ lv, const int32_t* 
     }
 }
 
-// the levels' weights are formed once per block (a division each), not once per cell
-__global__ void vbal_sub_T_kernel(double* __restrict__ lv, const int32_t* __restrict__ topo,
+// the levels' weights are formed once per block (a division each), not once per cell, VB_TILE levels at a time
+constexpr int VB_TILE = 128;
+__global__ void __launch_bounds__(VB_TILE) vbal_sub_T_kernel(double* __restrict__ lv, const int32_t* __restrict__ topo,
                                   const double* __restrict__ rs, const double* __restrict__ rad,
                                   int im, int jm, int km, int KP, double dr, int zonal) {
-    extern __shared__ double wgt[];
-    for (int i = threadIdx.x; i < im; i += blockDim.x)
-        wgt[i] = vbal_weight(rad, i, im, dr, vbal_I0(rad, im, dr));
-    __syncthreads();
+    __shared__ double wgt[VB_TILE];
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y + 1;
-    if (k >= km || topo[(size_t)j * km + k] != 0) return;
     const size_t plane = (size_t)jm * KP, b = (size_t)j * KP + k;
-    double S;
-    if (zonal) {
-        if (k >= km - 1 || rs[2 * j + 1] <= 0.0) return;    // not among the meridians averaged
-        S = rs[2 * j] / rs[2 * j + 1];
-    } else {
-        S = 0.0;
+    // zonal: only the meridians averaged
+    const bool on = k < km && topo[(size_t)j * km + k] == 0 && (!zonal || (k < km - 1 && rs[2 * j + 1] > 0.0));
+    const double I0 = vbal_I0(rad, im, dr);
+    double S = 0.0;
+    if (on && zonal) S = rs[2 * j] / rs[2 * j + 1];
+    else if (on)
         for (int i = 0; i < im; i++) S += lv[b + (size_t)i * plane];
-    }
+    for (int h = 0; h < im; h += VB_TILE) {
+        const int n = min(VB_TILE, im - h);
+        __syncthreads();
+        if (threadIdx.x < n) wgt[threadIdx.x] = vbal_weight(rad, h + threadIdx.x, im, dr, I0);
+        __syncthreads();
+        if (!on) continue;
 #pragma unroll 8
-    for (int i = 0; i < im; i++) lv[b + (size_t)i * plane] -= S * wgt[i];
+        for (int i = 0; i < n; i++) lv[b + (size_t)(h + i) * plane] -= S * wgt[i];
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -840,14 +843,19 @@ int bc_T(AtjupCtx* c, double* const a[LN]) {
     return ATJUP_OK;
 }
 
-int shapiro_T(AtjupCtx* c, double* const f[3]) {
+int shapiro_T(AtjupCtx* c, double* const* f, int n = 3) {
     const AtjupParams& P = c->P;
+    if ((long)P.im * n > MAX_GRID_Z) {         // as launch_shapiro_n
+        for (int x = 0; x < n; x++)
+            if (int rc = shapiro_T(c, f + x, 1)) return rc;
+        return ATJUP_OK;
+    }
     const FQ q = filt_q(c);
-    const dim3 grid((P.km + 127) / 128, P.jm, P.im * 3);
+    const dim3 grid((P.km + 127) / 128, P.jm, P.im * n);
     const int32_t *hk = c->floor_hi, *hj = c->floor_hi + (size_t)P.jm * c->KP;
     // scratch: the RK step's own stage buffers, rewritten by the next step
     TFields A{}, B{}, C{};
-    for (int x = 0; x < 3; x++) {
+    for (int x = 0; x < n; x++) {
         A.src[x] = f[x];
         A.dst[x] = c->X1[x];
         B.src[x] = c->X1[x];
@@ -872,7 +880,7 @@ int balance_T(AtjupCtx* c, double* lv) {
                                                           c->KP);
         c->launches++;
     }
-    vbal_sub_T_kernel<<<dim3((P.km + 127) / 128, P.jm - 2), 128, sizeof(double) * P.im, c->stream>>>(
+    vbal_sub_T_kernel<<<dim3((P.km + VB_TILE - 1) / VB_TILE, P.jm - 2), VB_TILE, 0, c->stream>>>(
         lv, c->topo, c->dvc, c->rad, P.im, P.jm, P.km, c->KP, P.dr, P.v_massbal_zonal);
     c->launches++;
     ATJUP_CHECK_LAUNCH("iteration adjoint: column balance");

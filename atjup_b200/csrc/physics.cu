@@ -151,10 +151,11 @@ __device__ __forceinline__ int precip_slot(int s) {
 // <float, double, float, float>.
 
 template <typename R> constexpr bool acc_free = sizeof(R) == 8;
-// Block shape and blocks per SM of the two stage kernels, which wait for memory: the more warps the better, until
-// the registers spill. Blocks of 128 threads, as a block's slot is held until its last warp ends and some
-// warps leave at once (solid cells, the rows by the poles). With the stage a template argument the species
-// fit 72 registers. 41x181x361, us a stage: 256 threads at 80 registers 282, 128 threads 265, then by stage 233
+// Block shape and blocks per SM of the two stage kernels, which wait for memory, by measurement: more warps
+// hide more of it, and spilled values cost some of that back. The FP64 species are fastest at 72 registers
+// (nothing spilt), the closure at 64, where all nine FP64 forms spill 96 to 116 bytes a thread. Blocks of
+// 128 threads, as a block's slot is held until its last warp ends and some warps leave at once (solid cells,
+// the rows by the poles). 41x181x361, us a stage: 256 threads at 80 registers 282, 128 threads 265, then by stage 233
 // at 80 registers, 224 at 72, 232 at 64; mixed (stages 0, 1, 3) 354, 265, 216 before, 222, 202, 179 at 64 and 217, 199,
 // 174 at 56. Closure 129 before, 134, 131, 123 at 80, 72, 64 and mixed 111, 100, 96.
 constexpr int PS_K = 64, PS_J = 2, CL_BLOCKS = 8;
@@ -282,7 +283,7 @@ __device__ __forceinline__ void species_all(const PhysStage& a, const Cell& x,
     }
 }
 
-// Bound by memory latency: about 440 bytes a cell, 4.3 TB/s at 282 us. (Species shared out over blocks: slower,
+// Bound by memory latency: about 440 bytes a cell, 5.3 TB/s at 224 us. (Species shared out over blocks: slower,
 // 319 us in two groups, 393 in four, as each group reads the shared fields again.)
 template <int ST, typename TI, typename TO, typename TA, typename R>
 __global__ void __launch_bounds__(PS_K * PS_J, SP_BLOCKS<R>) species_stage_kernel(PhysStage a) {

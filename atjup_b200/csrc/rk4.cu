@@ -832,12 +832,12 @@ static int make_box_map(CUtensorMap* m, const void* base, const AtjupCtx* c, int
     return ATJUP_OK;
 }
 
-// Radial planes per block of the stage kernel. A block's planes are a chain (3.7 us each when it has an
+// Radial planes per block of the stage kernel. A block's planes are a chain (2.3 us each when it has an
 // SM to itself), so a grid is cut into chunks short enough that every SM has its two blocks, down to
-// two planes (each chunk reads the two planes beside it again, from L2): 41x61x97, 27 tiles, 79 us a
-// stage in two chunks and 25 us in chunks of 4; 13x37x49, 12 tiles, 26 and 13 us. Grids that fill the
-// chip anyway take 8: chunks of 6 to 14 measured alike there (41x181x361: two dry iterations 1.80 to
-// 1.83 ms, 1.92 in two chunks, 2.01 in chunks of 2).
+// two planes (each chunk reads the two planes beside it again, from L2): 41x61x97, 27 tiles, 65 us a
+// stage in two chunks and 23 us in chunks of 4; 13x37x49, 12 tiles, 40 us in one chunk and 15 us in chunks of 2.
+// Grids that fill the chip anyway take 8: chunks of 4 to 21 measured alike there (41x181x361: 144 to 147 us a
+// stage, 171 in chunks of 2).
 static int planes_per_block(const AtjupParams& P) {
     const long tiles = (long)((P.km - 1 + TK - 1) / TK) * ((P.jm + TJ - 1) / TJ);
     int per = 8;

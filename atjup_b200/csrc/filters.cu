@@ -47,7 +47,7 @@ struct D2 {
 // takes k = 0's result of the k pass. Cells whose stencil lies wholly above the floor (i >= hi, the
 // highest floor of the columns within two cells along k, or along j) take the plain formula; the
 // others test each neighbour. Bound by the latency of the rows at 20 warps per SM (64 registers; 74 us at
-// 48, 78 us with the row loop unrolled to 122). u, v, w of the 41x181x361 shell: 57 us, 115 us in separate
+// 48, 78 us with the row loop unrolled to 122). u, v, w of the 41x181x361 shell: 52 us, 115 us in separate
 // k and j passes that tested the floor of every neighbour at every level.
 template <int ORDER>
 __global__ void __launch_bounds__(256, 4)
@@ -63,6 +63,8 @@ shapiro_kj_kernel(FiltFields F, const int32_t* __restrict__ topo, const int32_t*
     const double* __restrict__ src = f == 0 ? F.src[0] : f == 1 ? F.src[1] : F.src[2];
     double* __restrict__ dst = f == 0 ? F.dst[0] : f == 1 ? F.dst[1] : F.dst[2];
     const int j0 = blockIdx.y * rows, j1 = min(q.jm, j0 + rows);
+    pdl_next();
+    pdl_wait();
     auto order4 = [&](double vp2, double vp1, double cc, double vm1, double vm2) {
         const double d4 = vp2 - 4.0 * vp1 + 6.0 * cc - 4.0 * vm1 + vm2;
         return cc - q.c4 * d4;
@@ -154,6 +156,8 @@ shapiro_i_kernel(FiltFields F, const int32_t* __restrict__ topo, FiltConst q, in
     const size_t b = (size_t)j * q.KP + k;
     const double* __restrict__ x = (f == 0 ? F.src[0] : f == 1 ? F.src[1] : F.src[2]) + b;
     double* __restrict__ y = (f == 0 ? F.dst[0] : f == 1 ? F.dst[1] : F.dst[2]) + b;
+    pdl_next();
+    pdl_wait();
     const int sx = floor_at(topo, q.use_topo, j, k, q.km);
     const int sy = k == n ? sx : floor_at(topo, q.use_topo, j, k + 1, q.km);
     auto one = [&](int i, int is, double m2, double m1, double c, double p1, double p2) -> double {
@@ -306,23 +310,28 @@ int launch_shapiro_n(AtjupCtx* c, double* const* f, int n, int order, double str
     }
     const int pairs = (P.km - 1) / 2 + 1, th = std::min(256, (pairs + 31) / 32 * 32);
     const int kb = (pairs + th - 1) / th;
-    // rows and levels per thread: 15 (ORDER / 2 more are read on each side), fewer while the blocks do
-    // not fill the SMs
-    int rows = 15, per = 15;
-    while (rows > 5 && (long)kb * ((P.jm + rows - 1) / rows) * P.im * n < 8 * 148) rows -= 5;
-    while (per > 5 && (long)kb * P.jm * ((P.im + per - 1) / per) * n < 8 * 148) per -= 5;
+    // Rows and levels per thread (ORDER / 2 more are read on each side). A thread's are a chain of memory round
+    // trips, so few while the warps of one row each, which is what the SMs can hold about twice over at 12500,
+    // leave them idle; more where the reads beside a chunk are what counts. By a sweep of both over nine shells: one
+    // field of 9x21x33 23.3 us at 8 and 16.6 at 1 row, of 41x61x97 26.8 and 16.6, of 41x181x361 36.9 and 32.9 at 3 to 4
+    // (43.3 at 1), three fields of it 86.1 at 8 and 88.3 at 4; levels: 9x21x33 13.5 us at 1 and 16.5 at 5, 41x61x97
+    // 16.5 at both, 33x121x243 20.8 at 5, 23.8 at 1 and 24.8 at 15, three fields of 41x181x361 91.2 at 15, 92.1 at 5.
+    const long warps = (long)kb * (th / 32) * P.jm * P.im * n;
+    const int rows = (int)std::min(8L, (warps + 12499) / 12500);
+    const int per = warps <= 4000 ? 1 : warps <= 100000 ? 5 : 15;
+    // The launches overlap the tails of the kernels before them (launch_pdl) but for the largest: one field of 9x21x33
+    // 13.3 and 9.6 us so, of 41x61x97 16.4 and 12.6, of 41x181x361 32.8 and 28.7; with three of it too the
+    // iteration with physics, whose second stream then finds fewer free blocks, 7890 and 7975 us.
+    const bool overlap = warps <= 50000;
     const int chunks = (P.im + per - 1) / per;
     const dim3 gkj(kb, (P.jm + rows - 1) / rows, P.im * n), gi(kb, P.jm, n * chunks);
     const int32_t *hk = c->floor_hi, *hj = c->floor_hi + (size_t)P.jm * c->KP;
     for (int p = 0; p < passes; p++) {
         c->launches += 2;
-        if (order == 4) {
-            shapiro_kj_kernel<4><<<gkj, th, 0, c->stream>>>(there, c->topo, hk, hj, q, rows);
-            shapiro_i_kernel<4><<<gi, th, 0, c->stream>>>(back, c->topo, q, per, chunks);
-        } else {
-            shapiro_kj_kernel<2><<<gkj, th, 0, c->stream>>>(there, c->topo, hk, hj, q, rows);
-            shapiro_i_kernel<2><<<gi, th, 0, c->stream>>>(back, c->topo, q, per, chunks);
-        }
+        auto kj = order == 4 ? shapiro_kj_kernel<4> : shapiro_kj_kernel<2>;
+        auto ip = order == 4 ? shapiro_i_kernel<4> : shapiro_i_kernel<2>;
+        ATJUP_CUDA(launch_pdl(overlap, kj, gkj, th, 0, c->stream, there, c->topo, hk, hj, q, rows));
+        ATJUP_CUDA(launch_pdl(overlap, ip, gi, th, 0, c->stream, back, c->topo, q, per, chunks));
     }
     ATJUP_CHECK_LAUNCH("shapiro");
     return ATJUP_OK;
